@@ -28,6 +28,7 @@
 #include "jsd_common.cuh"
 #include "jsd_fft.cuh"
 #include "jsd_gemm.cuh"
+#include "jsd_parity.cuh"
 #include "jsd_spectral.cuh"
 #include "jsd_spectral_sq.cuh"
 #include "jsd_tc05.cuh"
@@ -210,6 +211,20 @@ struct jsd_plan {
   float *Dhi = nullptr, *Dlo = nullptr;  // TF32 split of D (mixed precision)
   bool mixed = false;
   double *Dm = nullptr, *VinvD = nullptr, *Vinv = nullptr, *Vfull = nullptr, *DVfull = nullptr;
+  // The operators on even and odd parts (jsd_parity.cuh), found by the whole
+  // operator they stand for; none when the tables have no definite parity or
+  // Ny is beyond the kernel's shapes
+  struct ParityOp {
+    const double* whole = nullptr;
+    size_t at[2] = {};
+    const double* a[2] = {};
+    int M[2] = {}, K[2] = {}, part[2] = {};
+    int kin = 0, mout = 0;
+    bool fold = false, unfold = false;
+  };
+  std::vector<ParityOp> par_ops;
+  int par_w = 0, par_tm = 0;  // kernel shape (0: no parity products)
+  int n_even = 0;             // even modes: eigen rows 0 .. n_even - 1
   double *lam = nullptr, *sgn = nullptr, *c0 = nullptr, *cN = nullptr, *w0 = nullptr, *wN = nullptr;
   double *yw = nullptr, *rhs_ns = nullptr, *lhs_inv_ns = nullptr, *ub = nullptr, *dub = nullptr;
   // workspace
@@ -473,8 +488,83 @@ void add_entry(GemmBatch& b, const double* A, const double* B, double* C, int M,
   e.alpha = alpha;
 }
 
+// f(W, TM, FOLD as integral constants) for a shape that parity_shape gives
+template <typename F>
+bool with_parity_shape(int w, int tm, F&& f) {
+  auto go = [&](auto W, auto TM) {
+    f(W, TM);
+    return true;
+  };
+#define JSD_SHAPE(a, b) \
+  if (w == a && tm == b) return go(std::integral_constant<int, a>{}, std::integral_constant<int, b>{})
+  JSD_SHAPE(1, 1);
+  JSD_SHAPE(2, 1);
+  JSD_SHAPE(3, 1);
+  JSD_SHAPE(2, 2);
+  JSD_SHAPE(5, 1);
+  JSD_SHAPE(2, 3);
+  JSD_SHAPE(4, 2);
+  JSD_SHAPE(3, 3);
+  JSD_SHAPE(5, 2);
+  JSD_SHAPE(6, 2);
+#undef JSD_SHAPE
+  return false;
+}
+
+// The batch on even and odd parts; false when an entry's operator has no such
+// form or the entries differ in what they fold.
+bool parity_batch(const jsd_plan* p, const GemmBatch& b, ParityBatch& o, bool& fold) {
+  if (!p->par_w || b.count < 1 || b.ldb != b.N || b.ldc != b.N) return false;
+  memset(&o, 0, sizeof(o));
+  o.N = b.N;
+  o.count = b.count;
+  for (int i = 0; i < b.count; ++i) {
+    const GemmEntry& g = b.e[i];
+    const jsd_plan::ParityOp* op = nullptr;
+    for (const auto& q : p->par_ops)
+      if (q.whole == g.A) op = &q;
+    if (!op || g.alpha != 1.0 || op->kin != g.K || op->mout != g.M) return false;
+    if (i == 0) {
+      fold = op->fold;
+      o.unfold = op->unfold;
+    } else if (fold != op->fold || (o.unfold != 0) != op->unfold) {
+      return false;
+    }
+    ParityEntry& e = o.e[i];
+    for (int h = 0; h < 2; ++h) {
+      e.a[h] = op->a[h];
+      e.M[h] = op->M[h];
+      e.K[h] = op->K[h];
+      e.part[h] = op->part[h];
+    }
+    e.B = g.B;
+    e.C = g.C;
+    e.kin = op->kin;
+    e.mout = op->mout;
+  }
+  return true;
+}
+
+int launch_parity(const jsd_plan* p, ParityBatch& o, bool fold, cudaStream_t s) {
+  o.rows = parity_rows(o, fold, parity_ksteps(p->par_w * p->par_tm));
+  const long long tiles = (long long)((o.N + kParN - 1) / kParN) * o.count;
+  with_parity_shape(p->par_w, p->par_tm, [&](auto W, auto TM) {
+    using Cfg = ParityCfg<decltype(W)::value, decltype(TM)::value>;
+    const int grid = (int)std::min<long long>(tiles, (long long)Cfg::MIN_BLOCKS * p->num_sms);
+    if (fold)
+      k_parity<decltype(W)::value, decltype(TM)::value, true><<<grid, Cfg::THREADS, Cfg::smem(o.rows), s>>>(o);
+    else
+      k_parity<decltype(W)::value, decltype(TM)::value, false><<<grid, Cfg::THREADS, Cfg::smem(o.rows), s>>>(o);
+  });
+  JSD_LAUNCHED("k_parity");
+  return 0;
+}
+
 int launch_gemm(const jsd_plan* p, const GemmBatch& b, int max_m, GemmSite site, cudaStream_t s) {
   ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, gemm_flops(b), s);
+  ParityBatch o;
+  bool fold = false;
+  if (parity_batch(p, b, o, fold)) return launch_parity(p, o, fold, s);
   return launch_gemm_cfg(p, b, max_m, p->gemm_cfg[site], s);
 }
 
@@ -902,8 +992,9 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
   }
   {
     GemmBatch b = gemm_batch(p);
-    add_entry(b, p->Vfull, p->vnt, (double*)v, ny, ni);
+    // (entries of one operator next to each other: k_parity loads it once)
     add_entry(b, p->DVfull, p->vnt, (double*)p->dvn, ny, ni);
+    add_entry(b, p->Vfull, p->vnt, (double*)v, ny, ni);
     add_entry(b, p->Vfull, p->omnt, (double*)p->om, ny, ni);
     rc = launch_eig(p, b, ny, kSiteEigOut, s);
     if (rc) return rc;
@@ -1027,6 +1118,21 @@ int set_smem_limits() {
       using Cfg = decltype(cfg);
       e = cudaFuncSetAttribute(k_dgemm_t<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::BYTES);
     });
+    JSD_CUDA(e);
+  }
+  {
+    cudaError_t e = cudaSuccess;
+    for (int rt = 1; rt <= 12; ++rt) {
+      int w = 0, tm = 0;
+      if (!parity_shape(rt, w, tm)) continue;
+      with_parity_shape(w, tm, [&](auto W, auto TM) {
+        for (const void* fn : {(const void*)k_parity<decltype(W)::value, decltype(TM)::value, true>,
+                               (const void*)k_parity<decltype(W)::value, decltype(TM)::value, false>}) {
+          const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+          if (r != cudaSuccess) e = r;
+        }
+      });
+    }
     JSD_CUDA(e);
   }
   JSD_CUDA(cudaFuncSetAttribute(k_mean_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -1236,8 +1342,19 @@ int jsd_autotune(jsd_plan* plan, void* stream) {
     }
     // eigenbasis sites of mixed plans: the Ozaki int8 kernel against the best DMMA tile
     if (rc == 0 && site != kSiteDfield && plan->oz_ready && plan->mixed) {
+      ParityBatch o;
+      bool fold = false;
+      if (parity_batch(plan, b, o, fold)) {
+        // what kernel 0 of the site runs
+        rc = launch_parity(plan, o, fold, s);
+        if (rc == 0 && cudaEventRecord(e0, s) != cudaSuccess) rc = fail(JSD_ERR_CUDA, "cudaEventRecord");
+        for (int r = 0; r < 5 && rc == 0; ++r) rc = launch_parity(plan, o, fold, s);
+        if (rc == 0 && (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+                        cudaEventElapsedTime(&best, e0, e1) != cudaSuccess))
+          rc = fail(JSD_ERR_CUDA, "autotune timing");
+      }
       plan->eig_ms[site][0] = best / 5.f;
-      rc = launch_ozaki(plan, b, s);  // warm-up
+      if (rc == 0) rc = launch_ozaki(plan, b, s);  // warm-up
       if (rc == 0 && cudaEventRecord(e0, s) != cudaSuccess) rc = fail(JSD_ERR_CUDA, "cudaEventRecord");
       for (int r = 0; r < 5 && rc == 0; ++r) rc = launch_ozaki(plan, b, s);
       float ms = 0.f;
@@ -1439,6 +1556,108 @@ int jsd_launches_per_step(const jsd_plan* plan) {
   return 3 * per_stage + (cmf ? 3 + 1 : 0);
 }
 
+}  // extern "C"
+
+namespace {
+
+// The eigenbasis tables of a plan with every eigenvector exactly even or odd
+// and the even modes first (the order of the eigen rows is the plan's own),
+// and D exactly odd under y -> -y. An eigenvector as a solver returns it has
+// the other parity mixed in at the level its eigenvalue's neighbour allows
+// (7e-11 at Ny = 129), D is odd to its own round-off (5e-15 of its largest
+// entry; its first rows are kept and mirrored, so rows still sum to zero).
+struct SymTables {
+  bool ok = false;
+  int n_even = 0;
+  std::vector<int> order;  // the caller's eigen index of each row
+  std::vector<double> D, V, Vinv, lam, sgn, c0, cN, w0, wN;
+};
+
+SymTables symmetric_tables(const jsd_desc* d) {
+  SymTables t;
+  const int ny = d->ny, n = ny - 2;
+  auto D = [&](int r, int c) { return d->D[(size_t)r * ny + c]; };
+  auto V = [&](int r, int c) { return d->V[(size_t)r * n + c]; };
+  auto W = [&](int r, int c) { return d->Vinv[(size_t)r * n + c]; };
+  double dmax = 0, vmax = 0, wmax = 0;
+  for (int i = 0; i < ny * ny; ++i) dmax = std::max(dmax, std::fabs(d->D[i]));
+  for (int i = 0; i < n * n; ++i) {
+    vmax = std::max(vmax, std::fabs(d->V[i]));
+    wmax = std::max(wmax, std::fabs(d->Vinv[i]));
+  }
+  std::vector<int>& order = t.order;
+  for (int want : {1, -1})
+    for (int j = 0; j < n; ++j)
+      if (d->sgn[j] == want) order.push_back(j);
+  if ((int)order.size() != n) return t;
+  for (int j = 0; j < n; ++j) t.n_even += d->sgn[j] == 1;
+  if (t.n_even != (n + 1) / 2) return t;
+  // (comparisons written so that a NaN fails them)
+  for (int r = 0; r < ny; ++r)
+    for (int c = 0; c < ny; ++c)
+      if (!(std::fabs(D(r, c) + D(ny - 1 - r, ny - 1 - c)) <= 1e-10 * dmax)) return t;
+  for (int r = 0; r < n; ++r)
+    for (int c = 0; c < n; ++c)
+      if (!(std::fabs(V(r, c) - d->sgn[c] * V(n - 1 - r, c)) <= 1e-8 * vmax) ||
+          !(std::fabs(W(r, c) - d->sgn[r] * W(r, n - 1 - c)) <= 1e-8 * wmax))
+        return t;
+  t.ok = true;
+  t.D.resize((size_t)ny * ny);
+  for (int r = 0; r < ny; ++r)
+    for (int c = 0; c < ny; ++c)
+      t.D[(size_t)r * ny + c] = 2 * r < ny - 1   ? D(r, c)
+                                : 2 * r > ny - 1 ? -D(ny - 1 - r, ny - 1 - c)
+                                                 : 0.5 * (D(r, c) - D(r, ny - 1 - c));
+  t.V.resize((size_t)n * n);
+  t.Vinv.resize((size_t)n * n);
+  for (int j = 0; j < n; ++j) {
+    const int o = order[j];
+    for (int r = 0; r < n; ++r) {
+      t.V[(size_t)r * n + j] = 0.5 * (V(r, o) + d->sgn[o] * V(n - 1 - r, o));
+      t.Vinv[(size_t)j * n + r] = 0.5 * (W(o, r) + d->sgn[o] * W(o, n - 1 - r));
+    }
+    for (auto m : {std::make_pair(&t.lam, d->lam), std::make_pair(&t.sgn, d->sgn), std::make_pair(&t.c0, d->c0),
+                   std::make_pair(&t.cN, d->cN), std::make_pair(&t.w0, d->w0), std::make_pair(&t.wN, d->wN)})
+      m.first->push_back(m.second[o]);
+  }
+  return t;
+}
+
+// `whole` (device) on even and odd parts; A: its host copy. The fragments go to
+// `pack`; the operator's pointers are offsets into it until place_parity_ops.
+void add_parity_op(jsd_plan* p, const double* whole, const double* A, int mout, int kin, bool fold, bool unfold,
+                   std::vector<double>& pack) {
+  const ParityHalves hv = parity_halves(A, mout, kin, fold, unfold, p->n_even);
+  jsd_plan::ParityOp op;
+  op.whole = whole;
+  op.kin = kin;
+  op.mout = mout;
+  op.fold = fold;
+  op.unfold = unfold;
+  for (int h = 0; h < 2; ++h) {
+    const std::vector<double> pk = parity_pack(hv.h[h], hv.M[h], hv.K[h], p->par_w * p->par_tm);
+    op.at[h] = pack.size();
+    pack.insert(pack.end(), pk.begin(), pk.end());
+    op.M[h] = hv.M[h];
+    op.K[h] = hv.K[h];
+    op.part[h] = hv.part[h];
+  }
+  p->par_ops.push_back(op);
+}
+
+int place_parity_ops(jsd_plan* p, const std::vector<double>& pack) {
+  double* dev = nullptr;
+  int rc = upload(p, &dev, pack.data(), pack.size());
+  if (rc) return rc;
+  for (auto& op : p->par_ops)
+    for (int h = 0; h < 2; ++h) op.a[h] = dev + op.at[h];
+  return 0;
+}
+
+}  // namespace
+
+extern "C" {
+
 int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
   if (!d || !out) return fail(JSD_ERR_ARG, "null argument");
   *out = nullptr;
@@ -1500,6 +1719,28 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     return fail(JSD_ERR_ARG, "FFT length must factor into 2, 3, 5, 7");
   }
   const int ny = d->ny, ni = ny - 2;
+  // Mixed plans under flow control keep the caller's tables and whole
+  // operators: there the products' round-off decides FP32 roundings, and dP/dx,
+  // a difference of flow rates over dt, shows them (1e-8 of it where it is small).
+  const SymTables sym = p->mixed && d->constant_mass_flux ? SymTables() : symmetric_tables(d);
+  const jsd_desc* given = d;
+  jsd_desc own = *d;  // the caller's description with the plan's own tables
+  if (sym.ok) {
+    own.D = sym.D.data();
+    own.V = sym.V.data();
+    own.Vinv = sym.Vinv.data();
+    own.lam = sym.lam.data();
+    own.sgn = sym.sgn.data();
+    own.c0 = sym.c0.data();
+    own.cN = sym.cN.data();
+    own.w0 = sym.w0.data();
+    own.wN = sym.wN.data();
+    d = &own;
+    p->n_even = sym.n_even;
+    if (!parity_shape(parity_row_tiles((ny + 1) / 2), p->par_w, p->par_tm) ||
+        ni < 4 * parity_ksteps(p->par_w * p->par_tm))
+      p->par_w = p->par_tm = 0;
+  }
   p->lda = (ny + 15) / 16 * 16;
   p->fdoubles = 2 * (size_t)ny * g.nk * nb;
   p->edoubles = 2 * (size_t)ni * g.nk * nb;
@@ -1565,7 +1806,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     std::vector<float> hi((size_t)ny * p->lda, 0.f), lo((size_t)ny * p->lda, 0.f);
     for (int r = 0; r < ny; ++r)
       for (int c = 0; c < ny; ++c) {
-        const double x = d->D[(size_t)r * ny + c];
+        const double x = given->D[(size_t)r * ny + c];
         const float h = tf32_round((float)x);
         hi[(size_t)r * p->lda + c] = h;
         lo[(size_t)r * p->lda + c] = tf32_round((float)(x - (double)h));
@@ -1573,8 +1814,19 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     JSD_TRY(upload(p, &p->Dhi, hi.data(), hi.size()));
     JSD_TRY(upload(p, &p->Dlo, lo.data(), lo.size()));
     // V^-1 D and V^-1 split the same way (eigenbasis-in products of the
-    // FP32-accurate nonlinear terms)
-    const double* eiA[2] = {VinvD.data(), d->Vinv};
+    // FP32-accurate nonlinear terms). These parts, like D's, come from the
+    // caller's own tables: the split's last bit would move with their round-off
+    std::vector<double> gVinv((size_t)ni * ni), gVinvD((size_t)ni * ny);
+    for (int i = 0; i < ni; ++i) {
+      const double* row = given->Vinv + (size_t)(sym.ok ? sym.order[i] : i) * ni;
+      std::copy(row, row + ni, gVinv.begin() + (size_t)i * ni);
+      for (int c = 0; c < ny; ++c) {
+        long double acc = 0;
+        for (int j = 0; j < ni; ++j) acc += (long double)row[j] * given->D[(size_t)(j + 1) * ny + c];
+        gVinvD[(size_t)i * ny + c] = (double)acc;
+      }
+    }
+    const double* eiA[2] = {gVinvD.data(), gVinv.data()};
     const int eiK[2] = {ny, ni};
     for (int k = 0; k < 2; ++k) {
       std::vector<float> eh((size_t)ni * p->lda, 0.f), el((size_t)ni * p->lda, 0.f);
@@ -1597,7 +1849,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     if (ny <= kTcM + 1) {
       p->tc_rows = ny;
       std::vector<float> ahi, alo;
-      tc05_pack_a(d->D, ny, ny, ny, tf32_round, ahi, alo);
+      tc05_pack_a(given->D, ny, ny, ny, tf32_round, ahi, alo);
       JSD_TRY(upload(p, &p->tc_ahi, ahi.data(), ahi.size()));
       JSD_TRY(upload(p, &p->tc_alo, alo.data(), alo.size()));
       for (int k = 0; k < 2; ++k) {
@@ -1607,7 +1859,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
       }
       if (ny > kTcM) {
         std::vector<double> xr(kTcKp, 0.0);
-        for (int c = 0; c < ny; ++c) xr[c] = d->D[(size_t)kTcM * ny + c];
+        for (int c = 0; c < ny; ++c) xr[c] = given->D[(size_t)kTcM * ny + c];
         JSD_TRY(upload(p, &p->tc_xrow, xr.data(), xr.size()));
       }
       // the tcgen05 kernel is the default (58 us per call against 86 us for
@@ -1628,6 +1880,14 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
   JSD_TRY(upload_padded(p, &p->Vinv, d->Vinv, ni, ni, p->lda));
   JSD_TRY(upload_padded(p, &p->Vfull, Vfull.data(), ny, ni, p->lda));
   JSD_TRY(upload_padded(p, &p->DVfull, DVfull.data(), ny, ni, p->lda));
+  std::vector<double> par_pack;
+  if (p->par_w) {
+    add_parity_op(p, p->Dm, d->D, ny, ny, true, true, par_pack);
+    add_parity_op(p, p->VinvD, VinvD.data(), ni, ny, true, false, par_pack);
+    add_parity_op(p, p->Vinv, d->Vinv, ni, ni, true, false, par_pack);
+    add_parity_op(p, p->Vfull, Vfull.data(), ny, ni, false, true, par_pack);
+    add_parity_op(p, p->DVfull, DVfull.data(), ny, ni, false, true, par_pack);
+  }
   if (ny <= kOzM + 1) {
     // int8 slice packs of the four eigenbasis operators (V^-1 D: K = Ny; V and
     // D V: M = Ny; at most one of M, K above 128). FP64 plans may select the
@@ -1716,11 +1976,19 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
       JSD_TRY(upload_padded(p, &p->Vfull_T, vfT.data(), ni, ny, p->lda));
       JSD_TRY(upload_padded(p, &p->DVfull_T, dvT.data(), ni, ny, p->lda));
       JSD_TRY(upload_padded(p, &p->D_T, dT.data(), ny, ny, p->lda));
+      if (p->par_w) {
+        add_parity_op(p, p->VinvD_T, vdT.data(), ny, ni, false, true, par_pack);
+        add_parity_op(p, p->Vinv_T, viT.data(), ni, ni, false, true, par_pack);
+        add_parity_op(p, p->Vfull_T, vfT.data(), ni, ny, true, false, par_pack);
+        add_parity_op(p, p->DVfull_T, dvT.data(), ni, ny, true, false, par_pack);
+        add_parity_op(p, p->D_T, dT.data(), ny, ny, true, true, par_pack);
+      }
       JSD_TRY(dev_alloc(p, (void**)&p->adj_conv, 3 * n2 * sizeof(double2)));
       JSD_TRY(dev_alloc(p, (void**)&p->adj_x00, n2 * sizeof(double2)));
       JSD_TRY(dev_alloc(p, (void**)&p->adj_ub, n2 * sizeof(double2)));
     }
   }
+  if (p->par_w) JSD_TRY(place_parity_ops(p, par_pack));
   if (d->base_u) JSD_TRY(upload(p, &p->ub, d->base_u, ny));
   if (d->base_du) JSD_TRY(upload(p, &p->dub, d->base_du, ny));
 
