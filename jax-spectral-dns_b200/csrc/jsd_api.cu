@@ -73,17 +73,27 @@ bool smooth_radix(int n) {
   return n == 1;
 }
 
-// sides S of the square FFT lengths S * S with register-resident kernels
-constexpr int kSquareSides[] = {3, 4, 5, 7, 10, 14};
+// Sides S of the square FFT lengths S * S with register-resident kernels: a side
+// is taken as soon as S * S >= 3 K + 1, since work goes with the square of the
+// length (49 modes: 81 instead of 100, x pass 24 against 30 us at 65 planes; 41:
+// 64 instead of 100, 12 against 22; 161: 256 instead of shared-memory passes of
+// 243, x pass 435 against 1127 us, z passes 318 against 548, at 145 planes).
+// Sides 11, 13 and 15 would need DFTs of 11 and 13 points, or 15 points per lane
+// in pairs. The mixed form keeps the lengths 9, 16, 25, 49, 100, 196: another
+// length rounds its FP32 transforms another way.
+constexpr int kSquareSides[] = {3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
 
-int square_side(int n) {
+bool mixed_side(int sd) { return sd <= 5 || sd == 7 || sd == 10 || sd == 14; }
+
+int square_side(int n, bool mixed) {
   for (int sd : kSquareSides)
-    if (sd * sd == n) return sd;
+    if (sd * sd == n && (!mixed || mixed_side(sd))) return sd;
   return 0;
 }
 
-// Call f(std::integral_constant<int, S>) for a supported square side S.
-template <typename F>
+// Call f(std::integral_constant<int, S>) for a supported square side S (C the
+// transforms' complex type).
+template <typename C, typename F>
 bool with_square_side(int sd, F&& f) {
   switch (sd) {
     case 3: f(std::integral_constant<int, 3>{}); return true;
@@ -92,15 +102,24 @@ bool with_square_side(int sd, F&& f) {
     case 7: f(std::integral_constant<int, 7>{}); return true;
     case 10: f(std::integral_constant<int, 10>{}); return true;
     case 14: f(std::integral_constant<int, 14>{}); return true;
-    default: return false;
+    default: break;
   }
+  if constexpr (sizeof(C) == sizeof(double2)) switch (sd) {
+      case 6: f(std::integral_constant<int, 6>{}); return true;
+      case 8: f(std::integral_constant<int, 8>{}); return true;
+      case 9: f(std::integral_constant<int, 9>{}); return true;
+      case 12: f(std::integral_constant<int, 12>{}); return true;
+      case 16: f(std::integral_constant<int, 16>{}); return true;
+      default: break;
+    }
+  return false;
 }
 
 // smallest square length with kernels, else the smallest 2,3,5,7-smooth one
-int choose_fft_size(int m) {
+int choose_fft_size(int m, bool mixed) {
   const int need = 3 * (m / 2) + 1;
   for (int sd : kSquareSides)
-    if (sd * sd >= need) return sd * sd;
+    if (sd * sd >= need && (!mixed || mixed_side(sd))) return sd * sd;
   int n = need;
   while (!smooth_radix(n)) ++n;
   return n;
@@ -753,15 +772,15 @@ int nonlinear(jsd_plan* p, const double2* state, const double2* uhist, int stage
   return p->mixed ? transforms<float2>(p, state, uhist, conv, s) : transforms<double2>(p, state, uhist, conv, s);
 }
 
-// x-pass variants: 0 register square FFT (S lanes per line), 1 half-split
-// register FFT (2 S lanes per line, even S, not the dual), 2 shared-memory FFT.
-// The S-lane form holds S points x 7 (11 for the dual) products per lane, more
-// than the register file in FP64 beyond S = 7.
+// x-pass variants. Mixed form: 0 register square FFT (S lanes per line), 1
+// half-split register FFT (2 S lanes per line, even S, not the dual). FP64 form:
+// 0 (S <= 7) and 1 both run k_xmid_park (the dual: 0, S <= 7, k_xmid_dual_sq).
+// 2 shared-memory FFT.
 bool xmid_available(const jsd_plan* p, int v) {
   const bool dual = p->desc.kind == JSD_KIND_DUAL;
   const int S = p->sqx;
   if (v == 0) return S && (p->mixed || S <= 7);
-  if (v == 1) return S && S % 2 == 0 && !dual;
+  if (v == 1) return S && !dual && (S % 2 == 0 || (!p->mixed && S > 7));
   if (v == 2) return smooth_radix(p->g.px) && (size_t)kXmidZB * p->g.px <= (size_t)kXmidEPT * kXmidThreads;
   return false;
 }
@@ -795,22 +814,25 @@ int launch_xmid(jsd_plan* p, int variant, C* inter, C* out3, cudaStream_t s) {
     return 0;
   }
   const C* tab = p->mixed ? (const C*)p->tsqx32 : (const C*)p->tsqx;
-  with_square_side(p->sqx, [&](auto side) {
+  with_square_side<C>(p->sqx, [&](auto side) {
     constexpr int S = decltype(side)::value;
-    if (variant == 0) {
-      constexpr int ZC = XmidSq<C, S>::ZC;
-      const dim3 grid((g.pz + ZC - 1) / ZC, ny);
-      if (dual)
-        k_xmid_dual_sq<C, S><<<grid, kSqWarps * 32, XmidSq<C, S>::smem(g, 2 * kZinvLines), s>>>(
+    constexpr bool F32 = sizeof(C) == sizeof(float2);
+    auto grid = [&](int zc) { return dim3((g.pz + zc - 1) / zc, ny); };
+    if (dual) {
+      if constexpr (F32 || S <= 7)
+        k_xmid_dual_sq<C, S><<<grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, 2 * kZinvLines), s>>>(
             g, tab, inter, out3, p->ub, p->dub);
-      else
-        k_xmid_sq<C, S><<<grid, kSqWarps * 32, XmidSq<C, S>::smem(g, kZinvLines), s>>>(g, tab, inter, out3, ub,
-                                                                                      dub, lam);
+    } else if constexpr (!F32) {
+      using P = XLineLanes<S>;
+      constexpr int ZC = XmidPark<P>::ZC;
+      k_xmid_park<P><<<(ny * g.pz + ZC - 1) / ZC, kSqWarps * 32, XmidPark<P>::smem(g), s>>>(g, tab, inter, out3, ub,
+                                                                                           dub);
+    } else if (variant == 0) {
+      k_xmid_sq<C, S><<<grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, kZinvLines), s>>>(
+          g, tab, inter, out3, ub, dub, lam);
     } else if constexpr (S % 2 == 0) {
-      constexpr int ZC = XmidH2<C, S>::ZC;
-      const dim3 grid((g.pz + ZC - 1) / ZC, ny);
-      k_xmid_h2<C, S><<<grid, kSqWarps * 32, XmidH2<C, S>::smem(g, kZinvLines), s>>>(g, tab, inter, out3, ub, dub,
-                                                                                    lam);
+      k_xmid_h2<C, S><<<grid(XmidH2<C, S>::ZC), kSqWarps * 32, XmidH2<C, S>::smem(g, kZinvLines), s>>>(
+          g, tab, inter, out3, ub, dub, lam);
     }
   });
   JSD_LAUNCHED("k_xmid_sq");
@@ -846,7 +868,7 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
     ProfScope ps(p, JSD_PROF_ZINV, bytes, s);
     if (p->sqz) {
       const C* tab = p->mixed ? (const C*)p->tsqz32 : (const C*)p->tsqz;
-      with_square_side(p->sqz, [&](auto side) {
+      with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
         const int per_block = kSqWarps * SqLane<S>::G;
         k_zinv_sq<C, S><<<(ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zinv_sq_smem<C, S>(), s>>>(
@@ -868,7 +890,7 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
     ProfScope ps(p, JSD_PROF_ZFWD, sizeof(C) * 3.0 * ny * K1 * g.pz + sizeof(double2) * 3.0 * fs, s);
     if (p->sqz) {
       const C* tab = p->mixed ? (const C*)p->tsqz32 : (const C*)p->tsqz;
-      with_square_side(p->sqz, [&](auto side) {
+      with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
         const int per_block = kSqWarps * SqLane<S>::G;
         k_zfwd_sq<C, S><<<(ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zfwd_sq_smem<C, S>(), s>>>(
@@ -1142,24 +1164,26 @@ int set_smem_limits() {
   JSD_CUDA(cudaFuncSetAttribute(k_tc05_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
   JSD_CUDA(cudaFuncSetAttribute(k_oz8_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
   cudaError_t err = cudaSuccess;
-  for (int sd : kSquareSides)
-    with_square_side(sd, [&](auto side) {
+  auto limit = [&](const void* fn) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (e != cudaSuccess) err = e;
+  };
+  for (int sd : kSquareSides) {
+    with_square_side<double2>(sd, [&](auto side) {
       constexpr int S = decltype(side)::value;
-      const void* fns[] = {(const void*)k_zinv_sq<double2, S>,      (const void*)k_zinv_sq<float2, S>,
-                           (const void*)k_zfwd_sq<double2, S>,      (const void*)k_zfwd_sq<float2, S>,
-                           (const void*)k_xmid_sq<double2, S>,      (const void*)k_xmid_sq<float2, S>,
-                           (const void*)k_xmid_dual_sq<double2, S>, (const void*)k_xmid_dual_sq<float2, S>};
-      if constexpr (S % 2 == 0) {
-        for (const void* fn : {(const void*)k_xmid_h2<double2, S>, (const void*)k_xmid_h2<float2, S>}) {
-          const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-          if (e != cudaSuccess) err = e;
-        }
-      }
-      for (const void* fn : fns) {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-        if (e != cudaSuccess) err = e;
-      }
+      for (const void* fn : {(const void*)k_zinv_sq<double2, S>, (const void*)k_zfwd_sq<double2, S>,
+                             (const void*)k_xmid_park<XLineLanes<S>>})
+        limit(fn);
+      if constexpr (S <= 7) limit((const void*)k_xmid_dual_sq<double2, S>);
     });
+    with_square_side<float2>(sd, [&](auto side) {
+      constexpr int S = decltype(side)::value;
+      for (const void* fn : {(const void*)k_zinv_sq<float2, S>, (const void*)k_zfwd_sq<float2, S>,
+                             (const void*)k_xmid_sq<float2, S>, (const void*)k_xmid_dual_sq<float2, S>})
+        limit(fn);
+      if constexpr (S % 2 == 0) limit((const void*)k_xmid_h2<float2, S>);
+    });
+  }
   JSD_CUDA(err);
   done = true;
   return 0;
@@ -1691,8 +1715,8 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
   g.mz = d->mz;
   g.kx_max = d->mx / 2;
   g.kz_max = d->mz / 2;
-  g.px = d->px_fft > 0 ? d->px_fft : choose_fft_size(d->mx);
-  g.pz = d->pz_fft > 0 ? d->pz_fft : choose_fft_size(d->mz);
+  g.px = d->px_fft > 0 ? d->px_fft : choose_fft_size(d->mx, p->mixed);
+  g.pz = d->pz_fft > 0 ? d->pz_fft : choose_fft_size(d->mz, p->mixed);
   g.nk = d->mx * d->mz;
   g.nb = nb;
   p->nb_max = nb;
@@ -1704,7 +1728,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
   g.c_fwd = std::sqrt((double)d->px_ref * (double)d->pz_ref) / (s * (double)g.px * (double)g.pz);
   p->dpdx_scale = std::sqrt(((double)d->px_ref * (two_pi / d->lx) * (two_pi / d->lx)) *
                             ((double)d->pz_ref * (two_pi / d->lz) * (two_pi / d->lz)));
-  if (!square_side(g.px) && (size_t)kXmidZB * g.px > (size_t)kXmidEPT * kXmidThreads) {
+  if (!square_side(g.px, p->mixed) && (size_t)kXmidZB * g.px > (size_t)kXmidEPT * kXmidThreads) {
     destroy(p);
     return fail(JSD_ERR_ARG, "x FFT length too large for the x-pass kernel (max " +
                                  std::to_string(kXmidEPT * kXmidThreads / kXmidZB) + ")");
@@ -1774,8 +1798,8 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
 
   JSD_TRY(upload(p, &p->twx, twx.data(), twx.size()));
   JSD_TRY(upload(p, &p->twz, twz.data(), twz.size()));
-  p->sqx = square_side(g.px);
-  p->sqz = square_side(g.pz);
+  p->sqx = square_side(g.px, p->mixed);
+  p->sqz = square_side(g.pz, p->mixed);
   p->xmid_variant = default_xmid_variant(p);
   // default tiles before any autotuning: the two-stage 48- or 64-row tile that
   // pads the call site's row count least (configurations 0 and 1)

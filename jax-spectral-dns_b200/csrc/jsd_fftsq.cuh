@@ -36,11 +36,66 @@ __host__ __device__ constexpr int sq_split(int s) {
 }
 
 __host__ __device__ constexpr bool sq_supported(int s) {
-  return s == 2 || s == 3 || s == 4 || s == 5 || s == 7 || s == 8 || sq_split(s) != 0;
+  return s == 2 || s == 3 || s == 4 || s == 5 || s == 7 || s == 8 || s == 9 || s == 16 || sq_split(s) != 0;
 }
 
 template <int R, bool INV, typename C>
 __host__ __device__ __forceinline__ void dft_reg(C* x);
+
+// cos and sin of 2 pi m / R, R = 9 and 16, for the twiddles inside dft_square
+template <int R>
+__host__ __device__ __forceinline__ void square_root_table(int m, double& c, double& s) {
+  if (R == 9) {
+    const double C[5] = {1.0, 0.76604444311897803520, 0.17364817766693034885, -0.5, -0.93969262078590838405};
+    const double S[5] = {0.0, 0.64278760968653932632, 0.98480775301220805937, 0.86602540378443864676,
+                         0.34202014332566873304};
+    c = C[m];
+    s = S[m];
+  } else {
+    const double C[10] = {1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.0,
+                          -0.38268343236508977173, -0.70710678118654752440, -0.92387953251128675613, -1.0,
+                          -0.92387953251128675613};
+    const double S[10] = {0.0, 0.38268343236508977173, 0.70710678118654752440, 0.92387953251128675613, 1.0,
+                          0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.0,
+                          -0.38268343236508977173};
+    c = C[m];
+    s = S[m];
+  }
+}
+
+// A * A points as A-point DFTs with twiddles between (A = 3, 4)
+template <int A, bool INV, typename C>
+__host__ __device__ __forceinline__ void dft_square(C* x) {
+  using Rl = typename real_of<C>::type;
+#pragma unroll
+  for (int n2 = 0; n2 < A; ++n2) {
+    C a[A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) a[n1] = x[A * n1 + n2];
+    dft_reg<A, INV>(a);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+      if (n2 * k1) {
+        double c, s;
+        square_root_table<A * A>(n2 * k1, c, s);
+        a[k1] = cmul(a[k1], cmake<C>((Rl)c, (Rl)(INV ? s : -s)));
+      }
+      x[A * k1 + n2] = a[k1];
+    }
+  }
+  C y[A * A];
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    C b[A];
+#pragma unroll
+    for (int n2 = 0; n2 < A; ++n2) b[n2] = x[A * k1 + n2];
+    dft_reg<A, INV>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < A; ++k2) y[k1 + A * k2] = b[k2];
+  }
+#pragma unroll
+  for (int k = 0; k < A * A; ++k) x[k] = y[k];
+}
 
 template <int A, int B, bool INV, typename C>
 __host__ __device__ __forceinline__ void dft_pfa(C* x) {
@@ -83,16 +138,27 @@ __host__ __device__ __forceinline__ void dft_reg(C* x) {
     dft8<INV>(x);
   } else if constexpr (R == 3 || R == 5 || R == 7) {
     dft_odd<R, INV>(x);
+  } else if constexpr (R == 9) {
+    dft_square<3, INV>(x);
+  } else if constexpr (R == 16) {
+    dft_square<4, INV>(x);
   } else {
     static_assert(sq_split(R) != 0, "unsupported register DFT length");
     dft_pfa<sq_split(R), R / sq_split(R), INV>(x);
   }
 }
 
-// Exchange-buffer elements per group (rows padded to S + 1 against bank conflicts).
+// Exchange buffer of a group: rows an odd number of elements apart (16-byte
+// elements of one column then fall on distinct slots; S + 1 would put all seven
+// rows of S = 7 on one), and with three and more groups per warp groups S more
+// than a multiple of 16 apart, so that the lanes of a warp write one run of slots.
+template <int S>
+__host__ __device__ constexpr int sq_row() {
+  return S | 1;
+}
 template <int S>
 __host__ __device__ constexpr int sq_xbuf() {
-  return S * (S + 1);
+  return S * sq_row<S>() + (S <= 10 ? ((S - S * sq_row<S>()) % 16 + 16) % 16 : 0);
 }
 
 // Stage 1 of a transform of the line held by the S lanes of a group (t =
@@ -109,14 +175,14 @@ __host__ __device__ __forceinline__ void sq_stage1(C* x, const C* tw, C* xb, int
     x[j] = cmul(x[j], w);
   }
 #pragma unroll
-  for (int j = 0; j < S; ++j) xb[j * (S + 1) + t] = x[j];
+  for (int j = 0; j < S; ++j) xb[j * sq_row<S>() + t] = x[j];
 }
 
 // Stage 2: lane t reads row t and transforms it; x[m] = X[t + S m] on exit.
 template <int S, bool INV, typename C>
 __host__ __device__ __forceinline__ void sq_stage2(C* x, const C* xb, int t) {
 #pragma unroll
-  for (int j = 0; j < S; ++j) x[j] = xb[t * (S + 1) + j];
+  for (int j = 0; j < S; ++j) x[j] = xb[t * sq_row<S>() + j];
   dft_reg<S, INV>(x);
 }
 
@@ -150,7 +216,7 @@ __device__ __forceinline__ void sq_fft_tab(C* x, const C* tab, C* xb, int t, boo
       x[j] = cmul(x[j], w);
     }
 #pragma unroll
-    for (int j = 0; j < S; ++j) xb[j * (S + 1) + t] = x[j];
+    for (int j = 0; j < S; ++j) xb[j * sq_row<S>() + t] = x[j];
   }
   __syncwarp();
   if (live) sq_stage2<S, INV>(x, xb, t);
@@ -222,6 +288,160 @@ __device__ __forceinline__ void sq2_fft(C* x, const C* tab, C* xb, int t, int h,
   if (live) sq2_stage2<S, INV>(x, xb, tab, t, h);
   __syncwarp();
 }
+
+// Half-split form on lane pairs (S = 12, 14, 16): lane 2 t + h of a line holds
+// element positions t + S m, its partner the other half of column t.
+//   S = 2 H, H odd: prime-factor mapping, m = (H h + 2 r) mod S on entry and
+//     (H h + (H + 1) r) mod S on exit in register r: the split into H-point
+//     DFTs and pairs needs no twiddles.
+//   H even: m = 2 r + h both ways, twiddles w_S^r on the odd half as in sq2_fft.
+// The exchange buffer has 16 columns per row; column c of row j sits at
+// c ^ swizzle(j). The two rows a lane pair writes differ by 4 in the swizzle and
+// eight neighbouring rows have distinct ones, so the writes of eight lanes, and
+// the reads of eight rows (the lanes of a pair read the same entry), hit
+// distinct 16-byte slots. The twiddle table is swizzled likewise.
+template <int S>
+struct Sq2p {
+  static constexpr int H = S / 2, XS = 16;
+  static constexpr bool PF = H % 2 == 1;
+  static_assert(S == 12 || S == 14 || S == 16, "swizzles are laid out for these sides");
+  // m, and the exchange row, of register r in lane half h: m0 + (h ? step(m0) : 0)
+  static __host__ __device__ constexpr int out0(int r) { return PF ? (H + 1) * r % S : 2 * r; }
+  static __host__ __device__ constexpr int row0(int r) { return PF ? out0(r) : r; }
+  static __host__ __device__ constexpr int step(int m0) { return PF ? (m0 < H ? H : -H) : 1; }
+  static __host__ __device__ constexpr int rstep(int j0) { return PF ? step(j0) : H; }
+  // entry register of the element that leaves a transform in register r
+  static __host__ __device__ constexpr int entry(int r) { return PF ? (H + 1) / 2 * r % H : r; }
+  static __host__ __device__ constexpr bool second(int j) { return PF ? j % 2 == 1 : j >= H; }
+  static __host__ __device__ constexpr int swizzle(int j) {
+    const int e = !second(j) ? j : PF ? (j >= H ? j - H : j + H) : j - H;  // the first row of j's pair
+    const int f = PF ? (e < 8 ? e / 2 : (e - 6) / 2) : S == 12 ? (e < 4 ? e : e + 2) : e;
+    return second(j) ? f ^ 4 : f;
+  }
+  static __host__ __device__ constexpr int xbuf() { return S * XS; }
+  static __host__ __device__ constexpr int tab() { return S * XS; }
+};
+
+// Entry e of the swizzled twiddle table (Sq2p::tab entries): w_N^(t j) at j * 16 + (t ^ 4 second(j))
+template <int S, typename C>
+__host__ __device__ __forceinline__ C sq2p_table_entry(const C* __restrict__ table, int e) {
+  const int j = e / Sq2p<S>::XS, t = (e % Sq2p<S>::XS) ^ (Sq2p<S>::second(j) ? 4 : 0);
+  return t < S ? table[t * j] : cmake<C>(0, 0);
+}
+
+// First half: the H-point DFT over a lane's own values, ready for the pair.
+// wS (even H only): 1 for the even half, then w_S^k, k < H, for the odd one (no
+// branch on the half).
+template <int S, bool INV, typename C>
+__host__ __device__ __forceinline__ void sq2p_first(C* x, const C* wS, int h) {
+  using Q = Sq2p<S>;
+  dft_reg<Q::H, INV>(x);
+  if constexpr (!Q::PF) {
+#pragma unroll
+    for (int k = 1; k < Q::H; ++k) {
+      C w = wS[h * Q::H + k];
+      if (INV) w.y = -w.y;
+      x[k] = cmul(x[k], w);
+    }
+  }
+}
+
+// The pair's value for the row that lane half sg (+1, -1) writes, times its twiddle
+template <bool INV, typename C, typename Rl>
+__host__ __device__ __forceinline__ C sq2p_pair(C own, C other, C w, Rl sg) {
+  if (INV) w.y = -w.y;
+  return cmul(cmake<C>(fma(sg, own.x, other.x), fma(sg, own.y, other.y)), w);
+}
+
+// Second half: x[n] = entry n0 of the row +- entry n1 (sq2p_n0, sq2p_n1), transformed
+template <int S>
+__host__ __device__ constexpr int sq2p_n0(int n) {
+  return Sq2p<S>::PF ? 2 * n : n;
+}
+template <int S>
+__host__ __device__ constexpr int sq2p_n1(int n) {
+  return Sq2p<S>::PF ? (S / 2 + 2 * n) % S : n + S / 2;
+}
+template <int S, bool INV, typename C>
+__host__ __device__ __forceinline__ void sq2p_second(C* x, const C* wS, int h) {
+  using Q = Sq2p<S>;
+  if constexpr (!Q::PF) {
+#pragma unroll
+    for (int n = 1; n < Q::H; ++n) {
+      C w = wS[h * Q::H + n];
+      if (INV) w.y = -w.y;
+      x[n] = cmul(x[n], w);
+    }
+  }
+  dft_reg<Q::H, INV>(x);
+}
+
+#if defined(__CUDACC__)
+// 16-byte shared-memory accesses by 32-bit address: an address with the line's
+// buffer on a 128-byte boundary takes a swizzle as an exclusive or
+// (volatile, so that they stay between the barriers of an exchange; table loads need not)
+__device__ __forceinline__ double2 lds16(unsigned a) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ double2 lds16_table(unsigned a) {
+  double2 v;
+  asm("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts16(unsigned a, double2 v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};\n" ::"r"(a), "d"(v.x), "d"(v.y));
+}
+
+// Shared-memory addresses of a lane: its column of the exchange rows (and of
+// the twiddle table) that its half writes, for rows whose step is +H or -H (or
+// the one step of even H), and its own row for reading, swizzles included
+struct Sq2pAddr {
+  unsigned wp, wm, tp, tm, row;
+};
+template <int S>
+__device__ __forceinline__ Sq2pAddr sq2p_addr(unsigned xb, unsigned tab, int t, int h) {
+  using Q = Sq2p<S>;
+  const unsigned th = 16u * (unsigned)(t ^ (h ? 4 : 0)), hs = h ? 16u * Q::XS * Q::H : 0u;
+  Sq2pAddr a;
+  a.wp = xb + th + hs;
+  a.tp = tab + th + hs;
+  a.wm = xb + th - hs;  // only used for rows of at least H
+  a.tm = tab + th - hs;
+  a.row = xb + 16u * (unsigned)(t * Q::XS + Q::swizzle(t));
+  return a;
+}
+
+template <int S, bool INV>
+__device__ __forceinline__ void sq2p_fft(double2* x, const double2* wS, const Sq2pAddr& ad, int h, bool live) {
+  using Q = Sq2p<S>;
+  constexpr unsigned ROW = 16u * Q::XS;
+  const double sg = h ? -1.0 : 1.0;
+  sq2p_first<S, INV>(x, wS, h);
+#pragma unroll
+  for (int k = 0; k < Q::H; ++k) {
+    double2 o;
+    o.x = __shfl_xor_sync(0xffffffffu, x[k].x, 1);
+    o.y = __shfl_xor_sync(0xffffffffu, x[k].y, 1);
+    const int j0 = Q::row0(k);
+    const bool up = Q::rstep(j0) > 0;
+    const double2 v = sq2p_pair<INV>(x[k], o, lds16_table((up ? ad.tp : ad.tm) + j0 * ROW), sg);
+    if (live) sts16(((up ? ad.wp : ad.wm) ^ (16u * Q::swizzle(j0))) + j0 * ROW, v);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int n = 0; n < Q::H; ++n) {
+    constexpr unsigned LOW = 7u;
+    const unsigned n0 = sq2p_n0<S>(n), n1 = sq2p_n1<S>(n);
+    const double2 b0 = lds16((ad.row ^ (16u * (n0 & LOW))) + 16u * (n0 & ~LOW));
+    const double2 b1 = lds16((ad.row ^ (16u * (n1 & LOW))) + 16u * (n1 & ~LOW));
+    x[n] = make_double2(fma(sg, b1.x, b0.x), fma(sg, b1.y, b0.y));
+  }
+  sq2p_second<S, INV>(x, wS, h);
+  __syncwarp();
+}
+#endif
 
 // Lane t's twiddles w_N^(t j), j = 1..S-1, from the table w_N^e, e = 0..N-1.
 template <int S, typename C>

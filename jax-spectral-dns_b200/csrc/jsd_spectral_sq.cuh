@@ -13,6 +13,8 @@
 // and the only synchronisation inside a transform is a __syncwarp.
 #pragma once
 
+#include <type_traits>
+
 #include "jsd_fftsq.cuh"
 #include "jsd_gemm.cuh"
 #include "jsd_spectral.cuh"
@@ -371,7 +373,8 @@ __device__ __forceinline__ void xsq_store(const Geo& g, const C* otile, C* __res
 }
 
 // Resident blocks per SM the FP32 x pass is compiled for (registers capped at
-// 168 per lane: a little spilling, 12 warps per SM instead of 8).
+// 168 per lane: a little spilling, 12 warps per SM instead of 8). The FP64 form
+// runs k_xmid_park.
 template <typename C>
 constexpr int xsq_min_blocks() {
   return sizeof(C) == sizeof(float2) ? 3 : 1;
@@ -547,8 +550,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_dual_sq(Geo g, const C* 
 
 // ---------------------------------------------------------------------------
 // x pass, half-split lanes (even S): a z column's lines on 2 S lanes, H = S / 2
-// points per lane (sq2_fft). Half the registers per lane of k_xmid_sq, so the
-// FP64 products fit without spilling.
+// points per lane (sq2_fft). Half the registers per lane of k_xmid_sq.
 // ---------------------------------------------------------------------------
 template <int S>
 struct SqLane2 {
@@ -717,6 +719,299 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __res
   }
   __syncthreads();
   xsq_store<C, ZC>(g, otile, out3, y, z0);
+}
+
+// ---------------------------------------------------------------------------
+// x pass of the FP64 form. The products take seven arrays per line besides the
+// line being transformed; what bounds the kernel is how many of them a lane
+// must hold (registers: warps in flight), then shared-memory wavefronts. So
+//  * the lines are paired by velocity component: (u, du/dx), (dv/dx, dw/dx),
+//    then (v, dv/dy), (du/dy, dw/dy), then (w, dw/dz), (du/dz, dv/dz); once a
+//    component has met its derivatives it goes to shared memory until the end
+//    and only four arrays live across a transform;
+//  * (u, du/dx) is one field times 1 - k (1 + k on the negative side): one load
+//    per position instead of two;
+//  * c_inv enters once, squared, at the end instead of scaling every line.
+// Lane policies: a line on S lanes (S points each), or, where 16 S registers
+// do not fit, on 2 S lanes (S / 2 points each, sq2p_fft).
+// Bound: shared-memory wavefronts (65% of the pipe at 129 x 129 modes, 129
+// planes, S = 14; FP64 pipe 34%, HBM 15%). Measured there 240 us, 344 us with
+// seven arrays live, lanes (t, h) at t + S h and branches on the mode range;
+// 33 x 33 modes x 776 planes (S = 7) 85 us from 163, 49 x 49 x 65 24 from 49
+// (S = 9 in place of 10), 161 x 161 x 145 435 from 1127 (S = 16 in place of
+// shared-memory passes of length 243).
+// ---------------------------------------------------------------------------
+template <int S_>
+struct LineFull {
+  static constexpr int S = S_, R = S, L = S, G = 32 / L, XB = sq_xbuf<S>(), TAB = S * sq_tw_stride(S);
+  // registers per thread: 4 arrays, the line and its temporaries (16 S + 20)
+  static constexpr int BLOCKS = S <= 5 ? 4 : S <= 9 ? 3 : 2;
+  static __device__ __forceinline__ int column(int li) { return li; }
+  static __device__ __forceinline__ int half(int) { return 0; }
+  static __device__ __forceinline__ int pos(int t, int, int r) { return t + S * r; }
+  // +1 where register r holds k >= 0 modes, -1 where k < 0 (K < N / 3: the
+  // positions between hold none)
+  static __device__ __forceinline__ double side(int, int r) { return 2 * r < S ? 1.0 : -1.0; }
+  static __device__ __forceinline__ constexpr int entry(int r) { return r; }
+  static __device__ __forceinline__ double2 twiddle(const double2* __restrict__ table, int e) {
+    const int j = e / sq_tw_stride(S), t = e % sq_tw_stride(S);
+    return t < S ? table[t * j] : make_double2(0.0, 0.0);
+  }
+  struct Addr {
+    const double2* tab;
+    double2* xb;
+  };
+  static __device__ __forceinline__ Addr addr(double2* xb, const double2* tab, int, int) { return {tab, xb}; }
+  static __device__ __forceinline__ void settle(Addr&) {}
+  template <bool INV>
+  static __device__ __forceinline__ void fft(double2* x, const double2*, const Addr& a, int t, int, bool live) {
+    sq_fft_tab<S, INV>(x, a.tab + sq_tw_stride(S), a.xb, t, live);
+  }
+};
+
+template <int S_>
+struct LineHalf {
+  using Q = Sq2p<S_>;
+  static constexpr int S = S_, R = S / 2, L = 2 * S, G = 32 / L, XB = Q::xbuf(), TAB = Q::tab();
+  static constexpr int BLOCKS = 3;
+  static __device__ __forceinline__ int column(int li) { return li >> 1; }
+  static __device__ __forceinline__ int half(int li) { return li & 1; }
+  static __device__ __forceinline__ int pos(int t, int h, int r) {
+    const int m = Q::out0(r);
+    return t + S * (m + (h ? Q::step(m) : 0));
+  }
+  static __device__ __forceinline__ double side(int h, int r) {
+    const int m = Q::out0(r);
+    if (!Q::PF) return 2 * m < S ? 1.0 : -1.0;
+    return (2 * m < S) == (h == 0) ? 1.0 : -1.0;
+  }
+  static __device__ __forceinline__ constexpr int entry(int r) { return Q::entry(r); }
+  static __device__ __forceinline__ double2 twiddle(const double2* __restrict__ table, int e) {
+    return sq2p_table_entry<S>(table, e);
+  }
+  using Addr = Sq2pAddr;
+  static __device__ __forceinline__ Addr addr(double2* xb, const double2* tab, int t, int h) {
+    return sq2p_addr<S>((unsigned)__cvta_generic_to_shared(xb), (unsigned)__cvta_generic_to_shared(tab), t, h);
+  }
+  // ties the table's addresses to this place: its loads do not move above it
+  // (nor are they kept in registers from one transform to the next)
+  static __device__ __forceinline__ void settle(Addr& a) { asm volatile("" : "+r"(a.tp), "+r"(a.tm)); }
+  template <bool INV>
+  static __device__ __forceinline__ void fft(double2* x, const double2* wS, const Addr& a, int, int h, bool live) {
+    sq2p_fft<S, INV>(x, wS, a, h, live);
+  }
+};
+
+template <int S>
+using XLineLanes = std::conditional_t<(S <= 10), LineFull<S>, LineHalf<S>>;
+
+template <class P>
+struct XmidPark {
+  static constexpr int S = P::S, ZC = kSqWarps * P::G;
+  // Input tile [zl][kx][field]: the nine fields of a mode lie together, so a
+  // line's reads along kx step over an odd number of 16-byte slots and a
+  // field is a fixed offset. kp rows per column, ZERO rows of zeros after the
+  // modes for the positions that have none (lane pairs pick the one four slots
+  // from the partner's mode); the staging copies of 8 threads (4 or 8 columns)
+  // hit distinct slots. The output tile [field][zl][kx] takes its place.
+  static constexpr int ZERO = P::L > S ? 8 : 1;
+  static __host__ __device__ int kp(int k1) {
+    return ZC == 4 ? k1 + ZERO + ((2 - ZERO - k1) % 8 + 8) % 8 : (k1 + ZERO) | 1;
+  }
+  static size_t smem(const Geo& g) {
+    return sizeof(double2) * ((size_t)kZinvLines * ZC * kp(g.kx_max + 1) + (size_t)ZC * P::XB + P::TAB + S) +
+           sizeof(double) * 2 * (size_t)ZC * P::R * P::L;
+  }
+};
+
+// Columns of the pass, plane after plane: a block's ZC columns may span two
+// planes, so a box narrower than ZC leaves no lanes idle. Offset of column c
+// in a field of the intermediate ([y][kx][z]); y = c / pz.
+__device__ __forceinline__ size_t xpark_column(const Geo& g, int c, int& y) {
+  y = c / g.pz;
+  return (size_t)y * (g.kx_max + 1) * g.pz + (c - y * g.pz);
+}
+
+// Asynchronous copies of the input tile
+template <int ZC, int ZERO>
+__device__ __forceinline__ void xpark_stage(const Geo& g, const double2* __restrict__ inter, double2* tile, int c0,
+                                            int kp) {
+  constexpr int RSTEP = kSqWarps * 32 / ZC;
+  const int K1 = g.kx_max + 1;
+  if (threadIdx.x < RSTEP * ZC) {
+    const int zl = threadIdx.x % ZC;
+    const bool ok = c0 + zl < g.ny * g.pz;
+    int y;
+    const double2* src = inter + (ok ? xpark_column(g, c0 + zl, y) : 0);
+    const size_t fstride = (size_t)g.ny * K1 * g.pz;
+    for (int kx = threadIdx.x / ZC; kx < K1; kx += RSTEP) {
+      const double2* s = src + (size_t)kx * g.pz;
+      double2* d = tile + (zl * kp + kx) * kZinvLines;
+#pragma unroll
+      for (int f = 0; f < kZinvLines; ++f) cp_async_elem(d + f, s + f * fstride, ok);
+    }
+  }
+  cp_async_commit();
+  constexpr int Z = ZERO * kZinvLines;
+  for (int i = threadIdx.x; i < ZC * Z; i += blockDim.x)
+    tile[((i / Z) * kp + K1) * kZinvLines + i % Z] = make_double2(0.0, 0.0);
+}
+
+enum XLine { kOwnDx, kBothDx, kPlain };  // (a, da/dx), (da/dx, db/dx), (a, b)
+
+// One position of a packed line a + i b at signed wavenumber k = side |k|:
+// a + i b for k >= 0, conj(a) + i conj(b) for k < 0 (k = 0: a, b are real)
+template <XLine KIND, int FA, int FB>
+__device__ __forceinline__ double2 xpark_value(const double2* mode, double side, double k) {
+  const double2 A = mode[FA];
+  if (KIND == kOwnDx) return make_double2(A.x * (1.0 - k), side * A.y * (1.0 - k));
+  const double2 B = mode[FB];
+  const double2 v = make_double2(fma(-side, B.y, A.x), fma(side, A.y, B.x));
+  return KIND == kPlain ? v : make_double2(-k * v.y, k * v.x);
+}
+
+template <class P>
+__global__ void __launch_bounds__(kSqWarps * 32, P::BLOCKS) k_xmid_park(Geo g, const double2* __restrict__ twtab,
+                                                                        const double2* __restrict__ inter,
+                                                                        double2* __restrict__ out3,
+                                                                        const double* __restrict__ ubase,
+                                                                        const double* __restrict__ dubase) {
+  using X = XmidPark<P>;
+  constexpr int S = P::S, N = S * S, R = P::R, G = P::G, ZC = X::ZC, XB = P::XB;
+  extern __shared__ __align__(128) unsigned char park_raw[];
+  const int K = g.kx_max, K1 = K + 1, KP = X::kp(K1);
+  double2* xball = reinterpret_cast<double2*>(park_raw);  // first: the swizzles want 128-byte boundaries
+  double2* tab = xball + ZC * XB;
+  double2* wS = tab + P::TAB;
+  double2* tile = wS + S;
+  double* park = reinterpret_cast<double*>(tile + kZinvLines * ZC * KP);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gi0 = lane / P::L, li = lane - gi0 * P::L;
+  const bool live = gi0 < G;
+  const int gi = live ? gi0 : 0;
+  const int h = live ? P::half(li) : 0, t = live ? P::column(li) : 0;
+  const int zl = warp * G + gi;
+  double2* xb = xball + zl * XB;
+  double* pk = park + (size_t)zl * 2 * R * P::L + (live ? li : 0);  // [2][R][L]
+  const int c0 = blockIdx.x * ZC, ncol = g.ny * g.pz;
+  xpark_stage<ZC, X::ZERO>(g, inter, tile, c0, KP);
+  for (int e = threadIdx.x; e < P::TAB; e += blockDim.x) tab[e] = P::twiddle(twtab, e);
+  if (threadIdx.x < S) wS[threadIdx.x] = 2 * threadIdx.x < S ? make_double2(1.0, 0.0) : twtab[(threadIdx.x - S / 2) * S];
+  // in units of c_inv: products of two fields take c_inv^2 at the end
+  const int yb = min(c0 + zl, ncol - 1) / g.pz / g.nb;
+  const double ub = ubase ? ubase[yb] / g.c_inv : 0.0, dub = dubase ? dubase[yb] / g.c_inv : 0.0;
+  const double c2 = g.c_inv * g.c_inv;
+  cp_async_wait<0>();
+  __syncthreads();
+  typename P::Addr ad = P::addr(xb, tab, t, h);
+  P::settle(ad);
+  // |mode| at each position, a zero row where there is none
+  auto mode_at = [&](int p) { return p <= K ? p : p >= N - K ? N - p : -1; };
+  int kxr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int kx = mode_at(P::pos(t, h, r));
+    kxr[r] = kx >= 0 ? kx : X::ZERO == 1 ? K1 : K1 + ((mode_at(P::pos(t, 1 - h, r)) + 4 - K1) & 7);
+  }
+  const double2* column = tile + zl * KP * kZinvLines;
+  auto line = [&](auto kind, auto fa, auto fb, double2* x) {
+    constexpr XLine KIND = decltype(kind)::value;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const double side = P::side(h, r);
+      x[P::entry(r)] = xpark_value<KIND, decltype(fa)::value, decltype(fb)::value>(
+          column + kxr[r] * kZinvLines, side, KIND == kPlain ? 0.0 : side * (kxr[r] * g.ax));
+    }
+    P::settle(ad);
+    P::template fft<true>(x, wS, ad, t, h, live);
+  };
+  using OwnDx = std::integral_constant<XLine, kOwnDx>;
+  using BothDx = std::integral_constant<XLine, kBothDx>;
+  using Plain = std::integral_constant<XLine, kPlain>;
+#define JSD_LINE(kind, fa, fb) line(kind{}, std::integral_constant<int, fa>{}, std::integral_constant<int, fb>{}, x)
+  // intermediate: 0 u, 1 v, 2 w, 3 du/dy, 4 dv/dy, 5 dw/dy, 6 du/dz, 7 dv/dz, 8 dw/dz
+  double2 x[R];
+  double A0[R], A1[R], A2[R], D[R], W[R];
+  JSD_LINE(OwnDx, 0, 0);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    W[r] = x[r].x + ub;  // U + u: the base flow advects like u
+    D[r] = x[r].y;
+    A0[r] = W[r] * x[r].y;
+    if (live) pk[r * P::L] = W[r];
+  }
+  JSD_LINE(BothDx, 1, 2);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    A1[r] = W[r] * x[r].x;
+    A2[r] = W[r] * x[r].y;
+  }
+  JSD_LINE(Plain, 1, 4);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    W[r] = x[r].x;
+    D[r] += x[r].y;
+    A1[r] = fma(W[r], x[r].y, A1[r]);
+    if (live) pk[(R + r) * P::L] = W[r];
+  }
+  JSD_LINE(Plain, 3, 5);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    A0[r] = fma(W[r], x[r].x, A0[r]);
+    A2[r] = fma(W[r], x[r].y, A2[r]);
+  }
+  JSD_LINE(Plain, 2, 8);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    W[r] = x[r].x;
+    D[r] += x[r].y;
+    A2[r] = fma(W[r], x[r].y, A2[r]);
+  }
+  JSD_LINE(Plain, 6, 7);
+#undef JSD_LINE
+  // hel_i = -(u . grad) u_i + (div u) u_i / 2 - U d_x u_i - delta_i0 (v U' - (div u) U / 2)
+  double2 z01[R], z2[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const double d = 0.5 * D[r], U = pk[r * P::L], V = pk[(R + r) * P::L];
+    const double a0 = fma(W[r], x[r].x, A0[r]), a1 = fma(W[r], x[r].y, A1[r]);
+    const double h0 = fma(-V, dub, fma(d, U, -a0)), h1 = fma(d, V, -a1), h2 = fma(d, W[r], -A2[r]);
+    z01[P::entry(r)] = make_double2(c2 * h0, c2 * h1);
+    z2[P::entry(r)] = make_double2(c2 * h2, 0.0);
+  }
+  P::template fft<false>(z01, wS, ad, t, h, live);
+  P::template fft<false>(z2, wS, ad, t, h, live);
+  __syncthreads();  // every line has read the input tile: outputs [f][zl][kx] take its place
+  if (live) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int p = P::pos(t, h, r);
+      xb[p] = z01[r];
+      if (p <= K) tile[(2 * ZC + zl) * KP + p] = z2[r];
+    }
+  }
+  __syncwarp();
+  if (live) {
+    for (int kx = li; kx <= K; kx += P::L) {
+      const double2 a = xb[kx], b = xb[kx == 0 ? 0 : N - kx];
+      // H0 = (Z[k] + conj Z[-k]) / 2, H1 = (Z[k] - conj Z[-k]) / (2 i)
+      tile[(0 * ZC + zl) * KP + kx] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
+      tile[(1 * ZC + zl) * KP + kx] = make_double2(0.5 * (a.y + b.y), -0.5 * (a.x - b.x));
+    }
+  }
+  __syncthreads();
+  constexpr int RSTEP = kSqWarps * 32 / ZC;
+  const int zs = threadIdx.x % ZC;
+  if (threadIdx.x < RSTEP * ZC && c0 + zs < ncol) {
+    int y;
+    double2* base = out3 + xpark_column(g, c0 + zs, y);
+    const size_t fstride = (size_t)g.ny * K1 * g.pz;
+    for (int kx = threadIdx.x / ZC; kx < K1; kx += RSTEP) {
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+        base[f * fstride + (size_t)kx * g.pz] = tile[(f * ZC + zs) * KP + kx];
+    }
+  }
 }
 
 }  // namespace jsd

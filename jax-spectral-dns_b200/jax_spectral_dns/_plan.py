@@ -78,7 +78,7 @@ class StepPlan:
         d = _native.JsdDesc()
         d.mx, d.ny, d.mz = mx, ny, mz
         d.px_ref, d.pz_ref = int(phys_ref[0]), int(phys_ref[-1])
-        px, pz = fft_sizes if fft_sizes is not None else (device_fft_size(mx), device_fft_size(mz))
+        px, pz = fft_sizes if fft_sizes is not None else (device_fft_size(mx, precision), device_fft_size(mz, precision))
         d.px_fft, d.pz_fft = int(px), int(pz)
         self.fft_sizes = (int(px), int(pz))
         d.lx, d.lz = float(lx), float(lz)
