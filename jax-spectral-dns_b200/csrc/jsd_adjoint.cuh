@@ -34,6 +34,7 @@ namespace jsd {
 __global__ void k_reconstruct_adj(Geo g, const double2* __restrict__ lu, const double2* __restrict__ lw,
                                   double2* __restrict__ dv_bar, double2* __restrict__ om_bar,
                                   double2* __restrict__ x00_bar) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(t / g.nk);
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update_adj(
     double* __restrict__ hg_old, double* __restrict__ X1_bar, double* __restrict__ T0_bar,
     double* __restrict__ T1_bar, double* __restrict__ vt_bar, double* __restrict__ omt_bar,
     double* __restrict__ wall_out) {
+  pdl();
   __shared__ double red[kEigParts][4][kEigCols];
   const int N = 2 * g.nk;
   const int lane = threadIdx.x % kEigCols;
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(32 * kMeanFlowRows) k_mean_flow_adj(
     Geo g, const double* __restrict__ lrT, const double* __restrict__ liT, const double2* __restrict__ ubar,
     double dt_gamma, double dt_xi, double2* __restrict__ x00_out, double2* __restrict__ conv_bar,
     double2* __restrict__ conv_bar_prev) {
+  pdl();
   const int n2 = 2 * g.ny;
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * kMeanFlowRows + (threadIdx.x >> 5);
@@ -258,6 +261,7 @@ __global__ void k_linear_terms_adj(Geo g, const double* __restrict__ ubase, cons
                                    const double2* __restrict__ omb, const double2* __restrict__ vextra,
                                    const double2* __restrict__ x00, double2* __restrict__ lu,
                                    double2* __restrict__ lv, double2* __restrict__ lw, double2* __restrict__ dvb) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(t / g.nk);
@@ -316,6 +320,7 @@ __global__ void k_linear_terms_adj(Geo g, const double* __restrict__ ubase, cons
 }
 
 __global__ void k_add_field(size_t n, const double2* __restrict__ a, double2* __restrict__ out) {
+  pdl();
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
     out[t] = cadd(out[t], a[t]);
 }
@@ -326,6 +331,7 @@ __global__ void k_add_field(size_t n, const double2* __restrict__ a, double2* __
 // (Sym, the Hermitian part, is an orthogonal projection).
 __global__ void k_energy_grad(Geo g, const double2* __restrict__ f, const double* __restrict__ w, double scale2,
                               double2* __restrict__ out) {
+  pdl();
   const size_t fs = (size_t)g.ny * g.nk;
   const size_t total = 3 * fs;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {

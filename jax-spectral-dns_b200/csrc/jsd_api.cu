@@ -60,6 +60,25 @@ int fail(int code, const std::string& msg) {
       return fail(JSD_ERR_CUDA, std::string("launch ") + name + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Whether the calling thread's launches are programmatic (pdl, jsd_common.cuh):
+// set for the length of an entry point by ProgrammaticLaunches.
+thread_local bool g_programmatic = false;
+
+template <typename... P, typename... A>
+void run(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = g_programmatic ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // errors: JSD_LAUNCHED
+}
+
 constexpr double kAlpha[3] = {29.0 / 96.0, -3.0 / 40.0, 1.0 / 6.0};
 constexpr double kBeta[3] = {37.0 / 160.0, 5.0 / 24.0, 1.0 / 6.0};
 constexpr double kGamma[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
@@ -280,6 +299,24 @@ struct jsd_plan {
 
 namespace {
 
+// Programmatic launches hide the start of a kernel behind the one before: two
+// steps of 9 x 65 x 5 modes take 144 us instead of 232, 33 x 65 x 33 413 instead
+// of 474, 97 x 97 x 97 (0.9 M entries per field) 2305 instead of 2434. From
+// fields that no longer share the L2 on they lose (129 x 129 x 129, 2.1 M entries:
+// 4706 against 4593), and in a captured graph, whose nodes already follow each
+// other closely, they cost 1 us per node (270 nodes at 33 x 65 x 33: 1892 us
+// against 1630), so both keep plain order.
+constexpr size_t kProgrammaticMax = 1u << 20;  // entries per field, all runs
+
+struct ProgrammaticLaunches {
+  ProgrammaticLaunches(const jsd_plan* p, cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    g_programmatic = (size_t)p->g.ny * p->g.nk * p->g.nb <= kProgrammaticMax &&
+                     cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  }
+  ~ProgrammaticLaunches() { g_programmatic = false; }
+};
+
 int dev_alloc(jsd_plan* p, void** ptr, size_t bytes) {
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e != cudaSuccess) return fail(JSD_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -350,7 +387,7 @@ int launch_gemm_cfg(const jsd_plan* p, const GemmBatch& b, int max_m, int cfg, c
   with_dgemm_cfg(cfg, [&](auto c) {
     using Cfg = decltype(c);
     const dim3 grid((b.N + Cfg::BN - 1) / Cfg::BN, (max_m + Cfg::BM - 1) / Cfg::BM, b.count);
-    k_dgemm_t<Cfg><<<grid, Cfg::THREADS, Cfg::BYTES, s>>>(b);
+    run(k_dgemm_t<Cfg>, grid, Cfg::THREADS, Cfg::BYTES, s, b);
   });
   JSD_LAUNCHED("k_dgemm");
   return 0;
@@ -399,7 +436,7 @@ int launch_tc05(jsd_plan* p, const float* const* a_hi, const float* const* a_lo,
   b.count = count;
   const int tiles = (b.N + kTcN - 1) / kTcN * b.count;
   ProfScope ps(p, JSD_PROF_SGEMM, flops, s);
-  k_tc05_split<<<tiles < p->num_sms ? tiles : p->num_sms, kTcThreads, kTcSmem, s>>>(b, p->errflag, p->wait_limit);
+  run(k_tc05_split, tiles < p->num_sms ? tiles : p->num_sms, kTcThreads, kTcSmem, s, b, p->errflag, p->wait_limit);
   JSD_LAUNCHED("k_tc05_split");
   return 0;
 }
@@ -445,7 +482,7 @@ int launch_split_eig_in(jsd_plan* p, cudaStream_t s) {
   }
   ProfScope ps(p, JSD_PROF_SGEMM, flops, s);
   const dim3 grid((b.N + Sgemm3Smem::BN - 1) / Sgemm3Smem::BN, 1, b.count);
-  k_sgemm3<<<grid, Sgemm3Smem::THREADS, Sgemm3Smem::BYTES, s>>>(b);
+  run(k_sgemm3, grid, Sgemm3Smem::THREADS, Sgemm3Smem::BYTES, s, b);
   JSD_LAUNCHED("k_sgemm3");
   return 0;
 }
@@ -482,7 +519,7 @@ int launch_dfield(jsd_plan* p, const double* const* src, double* const* dst, int
   }
   ProfScope ps(p, JSD_PROF_SGEMM, 2.0 * ny * (double)ny * b.N * count, s);
   const dim3 grid((b.N + Sgemm3Smem::BN - 1) / Sgemm3Smem::BN, 1, b.count);
-  k_sgemm3<<<grid, Sgemm3Smem::THREADS, Sgemm3Smem::BYTES, s>>>(b);
+  run(k_sgemm3, grid, Sgemm3Smem::THREADS, Sgemm3Smem::BYTES, s, b);
   JSD_LAUNCHED("k_sgemm3");
   return 0;
 }
@@ -571,9 +608,9 @@ int launch_parity(const jsd_plan* p, ParityBatch& o, bool fold, cudaStream_t s) 
     using Cfg = ParityCfg<decltype(W)::value, decltype(TM)::value>;
     const int grid = (int)std::min<long long>(tiles, (long long)Cfg::MIN_BLOCKS * p->num_sms);
     if (fold)
-      k_parity<decltype(W)::value, decltype(TM)::value, true><<<grid, Cfg::THREADS, Cfg::smem(o.rows), s>>>(o);
+      run(k_parity<decltype(W)::value, decltype(TM)::value, true>, grid, Cfg::THREADS, Cfg::smem(o.rows), s, o);
     else
-      k_parity<decltype(W)::value, decltype(TM)::value, false><<<grid, Cfg::THREADS, Cfg::smem(o.rows), s>>>(o);
+      run(k_parity<decltype(W)::value, decltype(TM)::value, false>, grid, Cfg::THREADS, Cfg::smem(o.rows), s, o);
   });
   JSD_LAUNCHED("k_parity");
   return 0;
@@ -674,8 +711,7 @@ int launch_ozaki(const jsd_plan* pc, const GemmBatch& b, cudaStream_t s) {
   }
   const long long tiles = (long long)((o.N + kOzN - 1) / kOzN) * o.count;
   ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, gemm_flops(b), s);
-  k_oz8_gemm<<<(int)std::min<long long>(tiles, p->num_sms), kOzThreads, kOzSmem, s>>>(o, p->errflag,
-                                                                                       p->wait_limit);
+  run(k_oz8_gemm, (int)std::min<long long>(tiles, p->num_sms), kOzThreads, kOzSmem, s, o, p->errflag, p->wait_limit);
   JSD_LAUNCHED("k_oz8_gemm");
   return 0;
 }
@@ -704,6 +740,7 @@ Geo planes_of(const Geo& g) {
 // h_v = -D q - k^2 H1 (only for the nonlinear-term hook)
 __global__ void k_assemble_hv(Geo g, const double2* __restrict__ dq, const double2* __restrict__ h1,
                               double2* __restrict__ hv) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % g.nk);
@@ -740,11 +777,11 @@ int nonlinear(jsd_plan* p, const double2* state, const double2* uhist, int stage
     const int blk = 256;
     ProfScope ps(p, JSD_PROF_LINEAR, sizeof(double2) * 7.0 * fs, s);
     if (p->desc.kind == JSD_KIND_PERTURBATION)
-      k_linear_terms<kPerturbation><<<grid_for(fs, blk), blk, 0, s>>>(gp, u, v, w, dv_in, p->ub, p->dub,
-                                                                      p->q, p->H1, p->hg, conv);
+      run(k_linear_terms<kPerturbation>, grid_for(fs, blk), blk, 0, s, gp, u, v, w, dv_in, p->ub, p->dub, p->q,
+          p->H1, p->hg, conv);
     else
-      k_linear_terms<kDual><<<grid_for(fs, blk), blk, 0, s>>>(gp, u, v, w, dv_in, p->ub, p->dub, p->q,
-                                                              p->H1, p->hg, conv);
+      run(k_linear_terms<kDual>, grid_for(fs, blk), blk, 0, s, gp, u, v, w, dv_in, p->ub, p->dub, p->q, p->H1, p->hg,
+          conv);
     JSD_LAUNCHED("k_linear_terms");
     return 0;
   }
@@ -807,9 +844,9 @@ int launch_xmid(jsd_plan* p, int variant, C* inter, C* out3, cudaStream_t s) {
     const size_t sm = XmidSmem<C, kXmidZB>::bytes(g);
     const dim3 grid((g.pz + kXmidZB - 1) / kXmidZB, ny);
     if (dual)
-      k_xmid_dual<C, kXmidZB><<<grid, kXmidThreads, sm, s>>>(g, p->fx, twx, inter, out3, p->ub, p->dub);
+      run(k_xmid_dual<C, kXmidZB>, grid, kXmidThreads, sm, s, g, p->fx, twx, inter, out3, p->ub, p->dub);
     else
-      k_xmid<C, kXmidZB><<<grid, kXmidThreads, sm, s>>>(g, p->fx, twx, inter, out3, ub, dub, lam);
+      run(k_xmid<C, kXmidZB>, grid, kXmidThreads, sm, s, g, p->fx, twx, inter, out3, ub, dub, lam);
     JSD_LAUNCHED("k_xmid");
     return 0;
   }
@@ -820,19 +857,19 @@ int launch_xmid(jsd_plan* p, int variant, C* inter, C* out3, cudaStream_t s) {
     auto grid = [&](int zc) { return dim3((g.pz + zc - 1) / zc, ny); };
     if (dual) {
       if constexpr (F32 || S <= 7)
-        k_xmid_dual_sq<C, S><<<grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, 2 * kZinvLines), s>>>(
-            g, tab, inter, out3, p->ub, p->dub);
+        run(k_xmid_dual_sq<C, S>, grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, 2 * kZinvLines), s, g,
+            tab, inter, out3, p->ub, p->dub);
     } else if constexpr (!F32) {
       using P = XLineLanes<S>;
       constexpr int ZC = XmidPark<P>::ZC;
-      k_xmid_park<P><<<(ny * g.pz + ZC - 1) / ZC, kSqWarps * 32, XmidPark<P>::smem(g), s>>>(g, tab, inter, out3, ub,
-                                                                                           dub);
+      run(k_xmid_park<P>, (ny * g.pz + ZC - 1) / ZC, kSqWarps * 32, XmidPark<P>::smem(g), s, g, tab, inter, out3, ub,
+          dub);
     } else if (variant == 0) {
-      k_xmid_sq<C, S><<<grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, kZinvLines), s>>>(
-          g, tab, inter, out3, ub, dub, lam);
+      run(k_xmid_sq<C, S>, grid(XmidSq<C, S>::ZC), kSqWarps * 32, XmidSq<C, S>::smem(g, kZinvLines), s, g, tab,
+          inter, out3, ub, dub, lam);
     } else if constexpr (S % 2 == 0) {
-      k_xmid_h2<C, S><<<grid(XmidH2<C, S>::ZC), kSqWarps * 32, XmidH2<C, S>::smem(g, kZinvLines), s>>>(
-          g, tab, inter, out3, ub, dub, lam);
+      run(k_xmid_h2<C, S>, grid(XmidH2<C, S>::ZC), kSqWarps * 32, XmidH2<C, S>::smem(g, kZinvLines), s, g, tab,
+          inter, out3, ub, dub, lam);
     }
   });
   JSD_LAUNCHED("k_xmid_sq");
@@ -871,12 +908,12 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
       with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
         const int per_block = kSqWarps * SqLane<S>::G;
-        k_zinv_sq<C, S><<<(ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zinv_sq_smem<C, S>(), s>>>(
-            g, tab, src, inter);
+        run(k_zinv_sq<C, S>, (ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zinv_sq_smem<C, S>(), s, g, tab,
+            src, inter);
       });
       JSD_LAUNCHED("k_zinv_sq");
     } else {
-      k_zinv<C><<<dim3(K1, ny), 256, sm, s>>>(g, p->fz, twz, src, inter);
+      run(k_zinv<C>, dim3(K1, ny), 256, sm, s, g, p->fz, twz, src, inter);
       JSD_LAUNCHED("k_zinv");
     }
   }
@@ -893,12 +930,12 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
       with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
         const int per_block = kSqWarps * SqLane<S>::G;
-        k_zfwd_sq<C, S><<<(ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zfwd_sq_smem<C, S>(), s>>>(
-            g, tab, out3, p->q, p->H1, p->hg, conv);
+        run(k_zfwd_sq<C, S>, (ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zfwd_sq_smem<C, S>(), s, g, tab,
+            out3, p->q, p->H1, p->hg, conv);
       });
       JSD_LAUNCHED("k_zfwd_sq");
     } else {
-      k_zfwd<C><<<dim3(K1, ny), 128, sm, s>>>(g, p->fz, twz, out3, p->q, p->H1, p->hg, conv);
+      run(k_zfwd<C>, dim3(K1, ny), 128, sm, s, g, p->fz, twz, out3, p->q, p->H1, p->hg, conv);
       JSD_LAUNCHED("k_zfwd");
     }
   }
@@ -925,18 +962,18 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
   const int blk = 256;
   if (!p->coupling && p->desc.kind != JSD_KIND_NS) {
     if (p->desc.kind == JSD_KIND_PERTURBATION)
-      k_coupling_off<kPerturbation><<<grid_for(fs, blk), blk, 0, s>>>(gp, v, p->dub, p->H1, p->hg);
+      run(k_coupling_off<kPerturbation>, grid_for(fs, blk), blk, 0, s, gp, v, p->dub, p->H1, p->hg);
     else
-      k_coupling_off<kDual><<<grid_for(fs, blk), blk, 0, s>>>(gp, u, p->dub, p->H1, p->hg);
+      run(k_coupling_off<kDual>, grid_for(fs, blk), blk, 0, s, gp, u, p->dub, p->H1, p->hg);
     JSD_LAUNCHED("k_coupling_off");
   }
   if (p->src_hv) {
-    k_add_source<<<grid_for(fs, blk), blk, 0, s>>>(gp, p->src_hv, p->src_hg, p->src_00, p->H1, p->hg,
-                                                   p->conv + (size_t)st * 2 * gp.ny);
+    run(k_add_source, grid_for(fs, blk), blk, 0, s, gp, p->src_hv, p->src_hg, p->src_00, p->H1, p->hg,
+        p->conv + (size_t)st * 2 * gp.ny);
     JSD_LAUNCHED("k_add_source");
   }
   if (!p->om_valid) {
-    k_omega<<<grid_for(fs, blk), blk, 0, s>>>(gp, u, w, p->om);
+    run(k_omega, grid_for(fs, blk), blk, 0, s, gp, u, w, p->om);
     JSD_LAUNCHED("k_omega");
   }
   // eigenbasis transforms. In the mixed form the nonlinear terms q, H1, h_g
@@ -967,9 +1004,9 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
   }
   if (p->src_hv) {
     if (split_in)
-      k_add_source00<float><<<1, 128, 0, s>>>(g, p->Vinv, p->lda, p->src_hv, reinterpret_cast<float*>(p->X1));
+      run(k_add_source00<float>, 1, 128, 0, s, g, p->Vinv, p->lda, p->src_hv, reinterpret_cast<float*>(p->X1));
     else
-      k_add_source00<double><<<1, 128, 0, s>>>(g, p->Vinv, p->lda, p->src_hv, p->X1);
+      run(k_add_source00<double>, 1, 128, 0, s, g, p->Vinv, p->lda, p->src_hv, p->X1);
     JSD_LAUNCHED("k_add_source00");
   }
   {
@@ -990,13 +1027,13 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
     const int blocks = (N + kEigCols - 1) / kEigCols, rpp = eigen_update_rpp(ny);
     const size_t sm = eigen_update_smem(ny);
     if (split_in)
-      k_eigen_update<float><<<blocks, kEigCols * kEigParts, sm, s>>>(
-          g, t, sc, reinterpret_cast<const float*>(p->X1), reinterpret_cast<const float*>(p->T),
+      run(k_eigen_update<float>, blocks, kEigCols * kEigParts, sm, s, g, t, sc,
+          reinterpret_cast<const float*>(p->X1), reinterpret_cast<const float*>(p->T),
           reinterpret_cast<const float*>(p->T + E), vt, omt, (const double*)v, reinterpret_cast<float*>(p->hv_old),
           reinterpret_cast<float*>(p->hg_old), p->vnt, p->omnt, rpp);
     else
-      k_eigen_update<double><<<blocks, kEigCols * kEigParts, sm, s>>>(
-          g, t, sc, p->X1, p->T, p->T + E, vt, omt, (const double*)v, p->hv_old, p->hg_old, p->vnt, p->omnt, rpp);
+      run(k_eigen_update<double>, blocks, kEigCols * kEigParts, sm, s, g, t, sc, p->X1, p->T, p->T + E, vt, omt,
+          (const double*)v, p->hv_old, p->hg_old, p->vnt, p->omnt, rpp);
     JSD_LAUNCHED("k_eigen_update");
   }
   {
@@ -1008,8 +1045,8 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
     // per-run matrices: lr / lns point at run 0's stage-st matrices, the kernel offsets by run
     const double* lr = p->lr_ns + (size_t)st * n2 * n2;
     const dim3 grid((unsigned)((n2 + kMeanFlowRows - 1) / kMeanFlowRows), (unsigned)g.nb);
-    k_mean_flow_rows<<<grid, 32 * kMeanFlowRows, sizeof(double2) * 2 * n2, s>>>(
-        g, lr, lns, u, w, conv, conv_old, dpdx, p->dpdx_scale, dte * kGamma[st], dte * kXi[st], p->uw00);
+    run(k_mean_flow_rows, grid, 32 * kMeanFlowRows, sizeof(double2) * 2 * n2, s, g, lr, lns, u, w, conv, conv_old,
+        dpdx, p->dpdx_scale, dte * kGamma[st], dte * kXi[st], p->uw00);
     JSD_LAUNCHED("k_mean_flow_rows");
   }
   {
@@ -1021,7 +1058,7 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
     rc = launch_eig(p, b, ny, kSiteEigOut, s);
     if (rc) return rc;
   }
-  k_reconstruct<<<grid_for(fs, blk), blk, 0, s>>>(g, p->dvn, p->om, p->uw00, u, v, w, p->errflag);
+  run(k_reconstruct, grid_for(fs, blk), blk, 0, s, g, p->dvn, p->om, p->uw00, u, v, w, p->errflag);
   JSD_LAUNCHED("k_reconstruct");
   // the back-transform left V^-1 v, V^-1 omega_y and dv/dy of the new state
   p->ev_valid = p->om_valid = p->dv_valid = true;
@@ -1031,12 +1068,12 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
 int mass_flux(jsd_plan* p, double2* state, double* dpdx, cudaStream_t s) {
   const Geo& g = p->g;
   const size_t fs = (size_t)g.ny * g.nk;
-  k_plane_sums_sliced<<<dim3(g.ny, kSumSlices), 256, 0, s>>>(g, state, 1, 1, p->partial);
+  run(k_plane_sums_sliced, dim3(g.ny, kSumSlices), 256, 0, s, g, state, 1, 1, p->partial);
   JSD_LAUNCHED("k_plane_sums_sliced");
-  k_mass_flux_scalar_sliced<<<1, 32, 0, s>>>(g.ny, p->yw, p->partial, g.c_inv, p->desc.flow_rate_target,
-                                             p->desc.dt_explicit, dpdx, p->scal);
+  run(k_mass_flux_scalar_sliced, 1, 32, 0, s, g.ny, p->yw, p->partial, g.c_inv, p->desc.flow_rate_target,
+      p->desc.dt_explicit, dpdx, p->scal);
   JSD_LAUNCHED("k_mass_flux_scalar_sliced");
-  k_roundtrip_shift<<<grid_for(fs, 256), 256, 0, s>>>(g, state, p->scal, p->tmp);
+  run(k_roundtrip_shift, grid_for(fs, 256), 256, 0, s, g, state, p->scal, p->tmp);
   JSD_LAUNCHED("k_roundtrip_shift");
   JSD_CUDA(cudaMemcpyAsync(state, p->tmp, fs * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   p->om_valid = false;  // u changed; v (and so V^-1 v, dv/dy) did not
@@ -1057,7 +1094,7 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
   double2 *lu = lam, *lv = lam + fs, *lw = lam + 2 * fs;
   const int blk = 256;
   // 9'
-  k_reconstruct_adj<<<grid_for(fs, blk), blk, 0, s>>>(g, lu, lw, p->dvn, p->om, p->adj_ub);
+  run(k_reconstruct_adj, grid_for(fs, blk), blk, 0, s, g, lu, lw, p->dvn, p->om, p->adj_ub);
   JSD_LAUNCHED("k_reconstruct_adj");
   // 8': cotangents of V^-1 v (from v and from dv/dy) and of V^-1 omega_y
   {
@@ -1074,9 +1111,9 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
     StageCoef sc{kAlpha[st], kBeta[st], kGamma[st], kXi[st], p->desc.dt, p->desc.dt_explicit, p->desc.re_tau,
                  st == 0 ? 1 : 0};
     const int N = 2 * g.nk;
-    k_eigen_update_adj<<<(N + kEigCols - 1) / kEigCols, kEigCols * kEigParts, 0, s>>>(
-        g, t, sc, last ? 1 : 0, p->T + 0 * E, p->T + 1 * E, p->T + 2 * E, p->hv_old, p->hg_old, p->X1, p->T + 3 * E,
-        p->vnt, p->omnt, p->vnt_alt, (double*)p->tmp);
+    run(k_eigen_update_adj, (N + kEigCols - 1) / kEigCols, kEigCols * kEigParts, 0, s, g, t, sc, last ? 1 : 0,
+        p->T + 0 * E, p->T + 1 * E, p->T + 2 * E, p->hv_old, p->hg_old, p->X1, p->T + 3 * E, p->vnt, p->omnt,
+        p->vnt_alt, (double*)p->tmp);
     JSD_LAUNCHED("k_eigen_update_adj");
   }
   // 7'
@@ -1084,10 +1121,9 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
     const size_t n2 = 2 * (size_t)ny;
     const double dte = p->desc.dt_explicit;
     const unsigned grid = (unsigned)((n2 + kMeanFlowRows - 1) / kMeanFlowRows);
-    k_mean_flow_adj<<<grid, 32 * kMeanFlowRows, 0, s>>>(g, p->lr_T + (size_t)st * n2 * n2, p->li_T + (size_t)st * n2 * n2,
-                                                        p->adj_ub, dte * kGamma[st], dte * kXi[st], p->adj_x00,
-                                                        p->adj_conv + (size_t)st * n2,
-                                                        st > 0 ? p->adj_conv + (size_t)(st - 1) * n2 : nullptr);
+    run(k_mean_flow_adj, grid, 32 * kMeanFlowRows, 0, s, g, p->lr_T + (size_t)st * n2 * n2,
+        p->li_T + (size_t)st * n2 * n2, p->adj_ub, dte * kGamma[st], dte * kXi[st], p->adj_x00,
+        p->adj_conv + (size_t)st * n2, st > 0 ? p->adj_conv + (size_t)(st - 1) * n2 : nullptr);
     JSD_LAUNCHED("k_mean_flow_adj");
   }
   // 5': cotangents of q (all rows), H1, h_g, the interior of v and of omega_y
@@ -1104,9 +1140,8 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
   // 4' .. 2': the state cotangent but D^T dv_bar, and dv_bar
   {
     const size_t n2 = 2 * (size_t)ny;
-    k_linear_terms_adj<<<grid_for(fs, blk), blk, 0, s>>>(g, p->ub, p->dub, p->q, p->H1, p->hg,
-                                                        p->adj_conv + (size_t)st * n2, p->Dfld, p->tmp, p->adj_x00,
-                                                        lu, lv, lw, p->Dfld + fs);
+    run(k_linear_terms_adj, grid_for(fs, blk), blk, 0, s, g, p->ub, p->dub, p->q, p->H1, p->hg,
+        p->adj_conv + (size_t)st * n2, p->Dfld, p->tmp, p->adj_x00, lu, lv, lw, p->Dfld + fs);
     JSD_LAUNCHED("k_linear_terms_adj");
   }
   // 1': v_bar += D^T dv_bar
@@ -1116,7 +1151,7 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
     int rc = launch_gemm(p, b, ny, kSiteDfield, s);
     if (rc) return rc;
   }
-  k_add_field<<<grid_for(fs, blk), blk, 0, s>>>(fs, p->Dfld + 2 * fs, lv);
+  run(k_add_field, grid_for(fs, blk), blk, 0, s, fs, p->Dfld + 2 * fs, lv);
   JSD_LAUNCHED("k_add_field");
   return 0;
 }
@@ -2083,6 +2118,7 @@ int run_steps(jsd_plan* plan, double2* st, double* dpdx, int first_step, int n_s
 int jsd_step(jsd_plan* plan, void* state, double* dpdx, int first_step, int n_steps, void* stream) {
   if (!plan || !state || !dpdx || n_steps < 0) return fail(JSD_ERR_ARG, "null argument");
   plan->ev_valid = plan->om_valid = plan->dv_valid = false;  // the caller may have changed the state
+  const ProgrammaticLaunches pl(plan, static_cast<cudaStream_t>(stream));
   return run_steps(plan, static_cast<double2*>(state), dpdx, first_step, n_steps, static_cast<cudaStream_t>(stream));
 }
 
@@ -2090,6 +2126,7 @@ int jsd_step_trajectory(jsd_plan* plan, void* state, double* dpdx, int first_ste
                         void* stream) {
   if (!plan || !state || !dpdx || !states || n_steps < 0) return fail(JSD_ERR_ARG, "null argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const size_t bytes = 3 * (size_t)plan->g.ny * plan->g.nk * plan->g.nb * sizeof(double2);
   char* out = static_cast<char*>(states);
   JSD_CUDA(cudaMemcpyAsync(out, state, bytes, cudaMemcpyDeviceToDevice, s));
@@ -2106,6 +2143,7 @@ int jsd_correct_mass_flux(jsd_plan* plan, void* state, double* dpdx, void* strea
   if (!plan || !state) return fail(JSD_ERR_ARG, "null argument");
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   double* dp = dpdx ? dpdx : plan->scal + 1;  // a scratch slot when the caller keeps no pressure gradient
   plan->ev_valid = plan->om_valid = plan->dv_valid = false;
   return mass_flux(plan, static_cast<double2*>(state), dp, s);
@@ -2115,11 +2153,12 @@ int jsd_energy(jsd_plan* plan, const void* state, double* out, void* stream) {
   if (!plan || !state || !out) return fail(JSD_ERR_ARG, "null argument");
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const Geo& g = plan->g;
-  k_plane_sums_sliced<<<dim3(g.ny, kSumSlices), 256, 0, s>>>(g, static_cast<const double2*>(state), 3, 0,
-                                                              plan->partial);
+  run(k_plane_sums_sliced, dim3(g.ny, kSumSlices), 256, 0, s, g, static_cast<const double2*>(state), 3, 0,
+      plan->partial);
   JSD_LAUNCHED("k_plane_sums_sliced");
-  k_weighted_total_sliced<<<1, 32, 0, s>>>(g.ny, plan->yw, plan->partial, 0.25 * g.c_inv * g.c_inv, out);
+  run(k_weighted_total_sliced, 1, 32, 0, s, g.ny, plan->yw, plan->partial, 0.25 * g.c_inv * g.c_inv, out);
   JSD_LAUNCHED("k_weighted_total_sliced");
   return 0;
 }
@@ -2127,13 +2166,14 @@ int jsd_energy(jsd_plan* plan, const void* state, double* out, void* stream) {
 int jsd_energy_runs(jsd_plan* plan, const void* state, double* out, void* stream) {
   if (!plan || !state || !out) return fail(JSD_ERR_ARG, "null argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const Geo& g = plan->g;
   const Geo gp = planes_of(g);
-  k_plane_sums_sliced<<<dim3(gp.ny, kSumSlices), 256, 0, s>>>(gp, static_cast<const double2*>(state), 3, 0,
-                                                               plan->partial);
+  run(k_plane_sums_sliced, dim3(gp.ny, kSumSlices), 256, 0, s, gp, static_cast<const double2*>(state), 3, 0,
+      plan->partial);
   JSD_LAUNCHED("k_plane_sums_sliced");
-  k_weighted_total_runs_sliced<<<g.nb, 32, 0, s>>>(g.ny, g.nb, plan->yw, plan->partial, 0.25 * g.c_inv * g.c_inv,
-                                                    out);
+  run(k_weighted_total_runs_sliced, g.nb, 32, 0, s, g.ny, g.nb, plan->yw, plan->partial, 0.25 * g.c_inv * g.c_inv,
+      out);
   JSD_LAUNCHED("k_weighted_total_runs_sliced");
   return 0;
 }
@@ -2145,6 +2185,7 @@ int jsd_step_adjoint(jsd_plan* plan, void* cotangent, int n_steps, void* stream)
                              "mass-flux control");
   if (!plan->coupling) return fail(JSD_ERR_ARG, "the discrete adjoint needs coupling_term on");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const size_t n2 = 2 * (size_t)plan->g.ny;
   double2* lam = static_cast<double2*>(cotangent);
   for (int t = 0; t < n_steps; ++t) {
@@ -2163,10 +2204,11 @@ int jsd_energy_grad(jsd_plan* plan, const void* state, void* out, void* stream) 
   if (!plan || !state || !out) return fail(JSD_ERR_ARG, "null argument");
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const Geo& g = plan->g;
   const size_t total = 3 * (size_t)g.ny * g.nk;
-  k_energy_grad<<<grid_for(total, 256), 256, 0, s>>>(g, static_cast<const double2*>(state), plan->yw,
-                                                    0.5 * g.c_inv * g.c_inv, static_cast<double2*>(out));
+  run(k_energy_grad, grid_for(total, 256), 256, 0, s, g, static_cast<const double2*>(state), plan->yw,
+      0.5 * g.c_inv * g.c_inv, static_cast<double2*>(out));
   JSD_LAUNCHED("k_energy_grad");
   return 0;
 }
@@ -2202,11 +2244,12 @@ int jsd_flow_rate(jsd_plan* plan, const void* u_field, double* out, void* stream
   if (!plan || !u_field || !out) return fail(JSD_ERR_ARG, "null argument");
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const Geo& g = plan->g;
-  k_plane_sums_sliced<<<dim3(g.ny, kSumSlices), 256, 0, s>>>(g, static_cast<const double2*>(u_field), 1, 1,
-                                                              plan->partial);
+  run(k_plane_sums_sliced, dim3(g.ny, kSumSlices), 256, 0, s, g, static_cast<const double2*>(u_field), 1, 1,
+      plan->partial);
   JSD_LAUNCHED("k_plane_sums_sliced");
-  k_weighted_total_sliced<<<1, 32, 0, s>>>(g.ny, plan->yw, plan->partial, g.c_inv, out);
+  run(k_weighted_total_sliced, 1, 32, 0, s, g.ny, plan->yw, plan->partial, g.c_inv, out);
   JSD_LAUNCHED("k_weighted_total_sliced");
   return 0;
 }
@@ -2215,6 +2258,7 @@ int jsd_nonlinear_terms(jsd_plan* plan, const void* state, int time_step, void* 
   if (!plan || !state || !h_v || !h_g) return fail(JSD_ERR_ARG, "null argument");
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const ProgrammaticLaunches pl(plan, s);
   const Geo& g = plan->g;
   const size_t fs = (size_t)g.ny * g.nk;
   const double2* uhist = nullptr;
@@ -2231,7 +2275,7 @@ int jsd_nonlinear_terms(jsd_plan* plan, const void* state, int time_step, void* 
   add_entry(b, plan->Dm, (const double*)plan->q, (double*)plan->tmp, g.ny, g.ny);
   rc = launch_gemm(plan, b, g.ny, kSiteEigIn, s);
   if (rc) return rc;
-  k_assemble_hv<<<grid_for(fs, 256), 256, 0, s>>>(g, plan->tmp, plan->H1, static_cast<double2*>(h_v));
+  run(k_assemble_hv, grid_for(fs, 256), 256, 0, s, g, plan->tmp, plan->H1, static_cast<double2*>(h_v));
   JSD_LAUNCHED("k_assemble_hv");
   JSD_CUDA(cudaMemcpyAsync(h_g, plan->hg, fs * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   return 0;

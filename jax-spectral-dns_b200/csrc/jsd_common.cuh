@@ -74,6 +74,30 @@ __host__ __device__ __forceinline__ size_t sidx(const Geo& g, int y, int ix, int
   return ((size_t)y * g.mx + ix) * g.mz + iz;
 }
 
+// Programmatic launch order. The library launches its kernels with programmatic
+// stream serialisation: a kernel's blocks may start while the kernel before it
+// drains. Every kernel launched that way first waits for the kernels before it
+// (complete, their writes visible), then lets its own successor start; every
+// thread passes here before it touches memory that another kernel writes or
+// reads, so a kernel that is done implies that all before it are. In this order
+// at most the next kernel is resident early, and none starts while a kernel two
+// before it still fills caches. Only tables fixed at plan creation may be read
+// before the wait.
+__device__ __forceinline__ void pdl_trigger() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_wait() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl() {
+  pdl_wait();
+  pdl_trigger();
+}
+
 // `bytes` (a multiple of 16) from a 16-byte aligned global address into L2
 __device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
 #if defined(__CUDA_ARCH__)

@@ -69,6 +69,7 @@ struct DgemmCfg {
 
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS) k_dgemm_t(GemmBatch batch) {
+  pdl();
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, ST = Cfg::ST;
   constexpr int TM = Cfg::TM, TN = Cfg::TN, NT = Cfg::THREADS;
   extern __shared__ __align__(16) double gsm[];
@@ -239,6 +240,7 @@ __device__ __forceinline__ void mma_tf32(float* d, const unsigned* a, const unsi
 }
 
 __global__ void __launch_bounds__(Sgemm3Smem::THREADS) k_sgemm3(SplitGemmBatch batch) {
+  pdl();
   using S = Sgemm3Smem;
   constexpr int BN = S::BN, BK = S::BK, BM = S::BM;
   constexpr int TM = 3, TN = 4;

@@ -201,8 +201,8 @@ __global__ void __launch_bounds__(64 * W, ParityCfg<W, TM>::MIN_BLOCKS) k_parity
   const int N = batch.N;
   const int ntiles = (N + kParN - 1) / kParN;
   const long long total = (long long)ntiles * batch.count;
+  // (never empty: the grid has at most one CTA per tile)
   const int first = (int)(total * blockIdx.x / gridDim.x), last = (int)(total * (blockIdx.x + 1) / gridDim.x);
-  if (first >= last) return;
 
   const int bufd = batch.rows * BS;  // doubles per tile buffer
   double* xch = psm + 2 * bufd;      // [pass][W][...][32]
@@ -228,23 +228,29 @@ __global__ void __launch_bounds__(64 * W, ParityCfg<W, TM>::MIN_BLOCKS) k_parity
 
   double a[TM][KS], ax[TM];  // operand fragments; the extra column's entries of rows g
   const double* loaded = nullptr;
+  auto load_operator = [&](const ParityEntry& e) {
+    loaded = e.a[half];
+    const double* src = loaded + (size_t)w * TM * KS * 32 + lane;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+#pragma unroll
+      for (int s = 0; s < KS; ++s) a[i][s] = src[(i * KS + s) * 32];
+      ax[i] = loaded[RT * KS * 32 + (w * TM + i) * 8 + g];
+    }
+    for (int k = w * 32 + lane; k < e.K[half]; k += W * 32)
+      xas[half * (4 * KS + 4) + k] = loaded[RT * KS * 32 + 8 * RT + k];
+  };
   int ei = first / ntiles, n0 = (first - ei * ntiles) * kParN, buf = 0;
+  load_operator(batch.e[ei]);  // fixed at plan creation: needs no earlier kernel
+  pdl();
   load_tile(ei, n0, psm);
   for (int tile = first; tile < last; ++tile) {
     const double* Bs = psm + buf * bufd;
     const ParityEntry& e = batch.e[ei];
     const int M = e.M[half], K = e.K[half], kin = e.kin, mout = e.mout;
     if (e.a[half] != loaded) {
-      loaded = e.a[half];
-      const double* src = loaded + (size_t)w * TM * KS * 32 + lane;
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-#pragma unroll
-        for (int s = 0; s < KS; ++s) a[i][s] = src[(i * KS + s) * 32];
-        ax[i] = loaded[RT * KS * 32 + (w * TM + i) * 8 + g];
-      }
       __syncthreads();  // the extra rows of the last operator are no longer read
-      for (int k = w * 32 + lane; k < K; k += W * 32) xas[half * (4 * KS + 4) + k] = loaded[RT * KS * 32 + 8 * RT + k];
+      load_operator(e);
     }
     cp_async_wait<0>();
     __syncthreads();  // the tile is here, and every warp is done with the other buffer and with xch

@@ -43,6 +43,7 @@ struct ZinvSrc {
 
 template <typename C>
 __global__ void k_zinv(Geo g, FftDesc fz, const C* __restrict__ tw, ZinvSrc src, C* __restrict__ inter) {
+  pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char zsm_raw[];
   C* zsm = reinterpret_cast<C*>(zsm_raw);
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(kXmidThreads) k_xmid(Geo g, FftDesc fx, const 
                                                        const C* __restrict__ inter, C* __restrict__ out3,
                                                        const double* __restrict__ ubase,
                                                        const double* __restrict__ dubase, double lam_d) {
+  pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char xsm_raw[];
   C* xsm = reinterpret_cast<C*>(xsm_raw);
@@ -269,6 +271,7 @@ __global__ void __launch_bounds__(kXmidThreads) k_xmid_dual(Geo g, FftDesc fx, c
                                                             const C* __restrict__ inter, C* __restrict__ out3,
                                                             const double* __restrict__ ubase,
                                                             const double* __restrict__ dubase) {
+  pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char xsm_raw[];
   C* xsm = reinterpret_cast<C*>(xsm_raw);
@@ -372,6 +375,7 @@ __device__ __forceinline__ void write_terms(const Geo& g, int y, int ix, int iz,
 __global__ void k_add_source(Geo g, const double2* __restrict__ hv, const double2* __restrict__ hgs,
                              const double2* __restrict__ s00, double2* __restrict__ H1, double2* __restrict__ hg,
                              double2* __restrict__ conv00) {
+  pdl();
   const size_t n = (size_t)g.ny * g.nk, n00 = 2 * (size_t)g.ny;
   const size_t total = n > n00 ? n : n00;
   for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -400,6 +404,7 @@ __global__ void k_add_source(Geo g, const double2* __restrict__ hv, const double
 template <typename TI>
 __global__ void k_add_source00(Geo g, const double* __restrict__ vinv, int lda, const double2* __restrict__ hv,
                                TI* __restrict__ X1) {
+  pdl();
   const int n = g.ny - 2;
   const size_t N = 2 * (size_t)g.nk * g.nb;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -420,6 +425,7 @@ template <typename C>
 __global__ void k_zfwd(Geo g, FftDesc fz, const C* __restrict__ tw, const C* __restrict__ out3,
                        double2* __restrict__ q, double2* __restrict__ H1, double2* __restrict__ hg,
                        double2* __restrict__ conv00) {
+  pdl();
   extern __shared__ __align__(16) unsigned char fsm_raw[];
   C* fsm = reinterpret_cast<C*>(fsm_raw);
   const int pz = g.pz;
@@ -501,6 +507,7 @@ __global__ void k_linear_terms(Geo g, const double2* __restrict__ u, const doubl
                                const double* __restrict__ ubase, const double* __restrict__ dubase,
                                double2* __restrict__ q, double2* __restrict__ H1, double2* __restrict__ hg,
                                double2* __restrict__ conv00) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(t / g.nk);
@@ -533,6 +540,7 @@ __global__ void k_linear_terms(Geo g, const double2* __restrict__ u, const doubl
 template <int KIND>
 __global__ void k_coupling_off(Geo g, const double2* __restrict__ f, const double* __restrict__ dubase,
                                double2* __restrict__ H1, double2* __restrict__ hg) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(t / g.nk);
@@ -555,6 +563,7 @@ __global__ void k_coupling_off(Geo g, const double2* __restrict__ f, const doubl
 // omega_y = i kz u - i kx w (the y component of curl u, domain.py:920-933)
 __global__ void k_omega(Geo g, const double2* __restrict__ u, const double2* __restrict__ w,
                         double2* __restrict__ om) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % g.nk);
@@ -611,6 +620,7 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update(
     const TI* __restrict__ hgt, const double* __restrict__ vt, const double* __restrict__ omt,
     const double* __restrict__ vfield, TI* __restrict__ hv_old, TI* __restrict__ hg_old,
     double* __restrict__ vnt, double* __restrict__ omnt, int rpp) {
+  pdl();
   __shared__ double red[kEigParts][6][kEigCols];
   extern __shared__ double vps_all[];
   const int N = 2 * g.nk * g.nb;  // columns: real and imaginary parts of every mode of every run
@@ -730,6 +740,7 @@ __global__ void __launch_bounds__(kMeanFlowThreads) k_mean_flow(
     Geo g, const double* __restrict__ rhs_ns, const double* __restrict__ lhs_inv_ns, const double2* __restrict__ u,
     const double2* __restrict__ w, const double2* __restrict__ conv, const double2* __restrict__ conv_old,
     const double* __restrict__ dpdx, double dpdx_scale, double dt_gamma, double dt_xi, double2* __restrict__ uw00) {
+  pdl();
   extern __shared__ __align__(16) double2 msm[];
   const int n = g.ny, n2 = 2 * g.ny;
   // block = run of a batch: its matrices, its planes (y * nb + run) and conv entries
@@ -792,6 +803,7 @@ __global__ void __launch_bounds__(32 * kMeanFlowRows) k_mean_flow_rows(
     Geo g, const double* __restrict__ lr_ns, const double* __restrict__ lhs_inv_ns, const double2* __restrict__ u,
     const double2* __restrict__ w, const double2* __restrict__ conv, const double2* __restrict__ conv_old,
     const double* __restrict__ dpdx, double dpdx_scale, double dt_gamma, double dt_xi, double2* __restrict__ uw00) {
+  pdl();
   extern __shared__ __align__(16) double2 msm[];
   const int n = g.ny, n2 = 2 * g.ny;
   const int run = blockIdx.y, nb = g.nb;
@@ -836,6 +848,7 @@ __global__ void __launch_bounds__(32 * kMeanFlowRows) k_mean_flow_rows(
 __global__ void k_reconstruct(Geo g, const double2* __restrict__ dvn, const double2* __restrict__ omn,
                               const double2* __restrict__ uw00, double2* __restrict__ u, double2* __restrict__ v,
                               double2* __restrict__ w, int* __restrict__ err) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nb * g.nk;
   bool bad = false;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -915,6 +928,7 @@ constexpr int kSumSlices = 8;
 
 __global__ void __launch_bounds__(256) k_plane_sums_sliced(Geo g, const double2* __restrict__ f, int ncomp, int mode,
                                                           double* __restrict__ out) {
+  pdl();
   const int y = blockIdx.x, slice = blockIdx.y;
   const int chunk = (g.nk + kSumSlices - 1) / kSumSlices;
   const int r0 = slice * chunk, r1 = min(g.nk, r0 + chunk);
@@ -962,6 +976,7 @@ __device__ __forceinline__ double weighted_slices(int ny, int stride, int offset
 // out = scale * sum over planes (single run), one warp
 __global__ void k_weighted_total_sliced(int ny, const double* __restrict__ weights,
                                         const double* __restrict__ partial, double scale, double* __restrict__ out) {
+  pdl();
   const double a = weighted_slices(ny, 1, 0, weights, partial);
   if (threadIdx.x == 0) out[0] = scale * a;
 }
@@ -970,6 +985,7 @@ __global__ void k_weighted_total_sliced(int ny, const double* __restrict__ weigh
 __global__ void k_weighted_total_runs_sliced(int ny, int nb, const double* __restrict__ weights,
                                              const double* __restrict__ partial, double scale,
                                              double* __restrict__ out) {
+  pdl();
   const int run = blockIdx.x;
   const double a = weighted_slices(ny, nb, run, weights, partial);
   if (threadIdx.x == 0) out[run] = scale * a;
@@ -979,6 +995,7 @@ __global__ void k_weighted_total_runs_sliced(int ny, int nb, const double* __res
 __global__ void k_mass_flux_scalar_sliced(int ny, const double* __restrict__ weights,
                                           const double* __restrict__ partial, double c_inv, double q0, double dt_e,
                                           double* __restrict__ dpdx, double* __restrict__ qdiff) {
+  pdl();
   const double a = weighted_slices(ny, 1, 0, weights, partial);
   if (threadIdx.x == 0) {
     const double d = c_inv * a - q0;
@@ -991,6 +1008,7 @@ __global__ void k_mass_flux_scalar_sliced(int ny, const double* __restrict__ wei
 // (partial per plane from k_plane_sums).
 __global__ void k_weighted_total_runs(int ny, int nb, const double* __restrict__ weights,
                                       const double* __restrict__ partial, double scale, double* __restrict__ out) {
+  pdl();
   const int run = blockIdx.x * blockDim.x + threadIdx.x;
   if (run >= nb) return;
   double acc = 0.0;
@@ -1005,6 +1023,7 @@ __global__ void k_weighted_total_runs(int ny, int nb, const double* __restrict__
 __global__ void k_mass_flux_scalar(int ny, const double* __restrict__ weights, const double* __restrict__ partial,
                                    double c_inv, double q0, double dt_e, double* __restrict__ dpdx,
                                    double* __restrict__ qdiff) {
+  pdl();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double acc = 0.0;
     for (int y = 0; y < ny; ++y) acc += weights[y] * partial[y];
@@ -1017,6 +1036,7 @@ __global__ void k_mass_flux_scalar(int ny, const double* __restrict__ weights, c
 
 __global__ void k_roundtrip_shift(Geo g, const double2* __restrict__ f, const double* __restrict__ qdiff,
                                   double2* __restrict__ out) {
+  pdl();
   const size_t total = (size_t)g.ny * g.nk;
   const double shift = -qdiff[0] * 0.5 / g.c_inv;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {

@@ -62,6 +62,7 @@ __device__ __forceinline__ const double2* zinv_field(const ZinvSrc& src, int i) 
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __restrict__ twtab, ZinvSrc src,
                                                            C* __restrict__ inter) {
+  pdl();
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, XB = sq_xbuf<S>();
   // The two forms keep their best measured shapes: FP32 lines on half-warp
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zfwd_sq(Geo g, const C* __res
                                                            const C* __restrict__ out3, double2* __restrict__ q,
                                                            double2* __restrict__ H1, double2* __restrict__ hg,
                                                            double2* __restrict__ conv00) {
+  pdl();
   constexpr int N = S * S, XB = sq_xbuf<S>();
   extern __shared__ __align__(16) unsigned char sq_raw[];
   const SqLane<S> ln;
@@ -387,6 +389,7 @@ __global__ void __launch_bounds__(kSqWarps * 32, xsq_min_blocks<C>()) k_xmid_sq(
                                                            const C* __restrict__ inter, C* __restrict__ out3,
                                                            const double* __restrict__ ubase,
                                                            const double* __restrict__ dubase, double lam_d) {
+  pdl();
   using Rl = typename real_of<C>::type;
   constexpr int G = SqLane<S>::G, ZC = XmidSq<C, S>::ZC, XB = sq_xbuf<S>();
   extern __shared__ __align__(16) unsigned char sq_raw[];
@@ -481,6 +484,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_dual_sq(Geo g, const C* 
                                                                 const C* __restrict__ inter, C* __restrict__ out3,
                                                                 const double* __restrict__ ubase,
                                                                 const double* __restrict__ dubase) {
+  pdl();
   using Rl = typename real_of<C>::type;
   constexpr int G = SqLane<S>::G, ZC = XmidSq<C, S>::ZC, XB = sq_xbuf<S>();
   extern __shared__ __align__(16) unsigned char sq_raw[];
@@ -618,6 +622,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __res
                                                            const C* __restrict__ inter, C* __restrict__ out3,
                                                            const double* __restrict__ ubase,
                                                            const double* __restrict__ dubase, double lam_d) {
+  pdl();
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, H = S / 2, G = SqLane2<S>::G, ZC = XmidH2<C, S>::ZC, XB = sq_xbuf<S>();
   extern __shared__ __align__(16) unsigned char sq_raw[];
@@ -876,6 +881,7 @@ __global__ void __launch_bounds__(kSqWarps * 32, P::BLOCKS) k_xmid_park(Geo g, c
                                                                         double2* __restrict__ out3,
                                                                         const double* __restrict__ ubase,
                                                                         const double* __restrict__ dubase) {
+  pdl();
   using X = XmidPark<P>;
   constexpr int S = P::S, N = S * S, R = P::R, G = P::G, ZC = X::ZC, XB = P::XB;
   extern __shared__ __align__(128) unsigned char park_raw[];
