@@ -60,6 +60,48 @@ __global__ void k_reconstruct_adj(Geo g, const double2* __restrict__ lu, const d
   }
 }
 
+// 7'. Transpose of the (0,0) mean-flow update of stage s: x00_bar <- LR^T
+// ubar, f_bar = Linv^T ubar; conv_bar (this stage) -= dt_e gamma f_bar,
+// conv_bar_prev -= dt_e xi f_bar (null for the first stage). lrT / liT are the
+// stage's transposed matrices (2 Ny x 2 Ny, row-major). One warp per row of
+// the transposed product; the blocks lead the grid of k_eigen_update_adj, whose
+// work they do not touch.
+struct MeanFlowAdj {
+  const double *lrT, *liT;
+  const double2* ubar;
+  double dt_gamma, dt_xi;
+  double2 *x00_out, *conv_bar, *conv_bar_prev;
+  int blocks;
+};
+
+__device__ __forceinline__ void mean_flow_adj_block(const Geo& g, const MeanFlowAdj& m, int block) {
+  const int n2 = 2 * g.ny;
+  const int lane = threadIdx.x & 31;
+  const int i = block * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= n2) return;
+  const double* lr = m.lrT + (size_t)i * n2;
+  const double* li = m.liT + (size_t)i * n2;
+  double ax = 0.0, ay = 0.0, fx = 0.0, fy = 0.0;
+  for (int j = lane; j < n2; j += 32) {
+    const double2 b = m.ubar[j];
+    ax += lr[j] * b.x;
+    ay += lr[j] * b.y;
+    fx += li[j] * b.x;
+    fy += li[j] * b.y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    ax += __shfl_down_sync(0xffffffffu, ax, o);
+    ay += __shfl_down_sync(0xffffffffu, ay, o);
+    fx += __shfl_down_sync(0xffffffffu, fx, o);
+    fy += __shfl_down_sync(0xffffffffu, fy, o);
+  }
+  if (lane == 0) {
+    m.x00_out[i] = make_double2(ax, ay);
+    m.conv_bar[i] = csub(m.conv_bar[i], make_double2(m.dt_gamma * fx, m.dt_gamma * fy));
+    if (m.conv_bar_prev) m.conv_bar_prev[i] = csub(m.conv_bar_prev[i], make_double2(m.dt_xi * fx, m.dt_xi * fy));
+  }
+}
+
 // 6'. Transpose of k_eigen_update for one stage, one thread per real column
 // (same block shape as the forward kernel). Inputs: the cotangents of the new
 // V^-1 v (two parts, summed: from v and from dv/dy) and of the new V^-1
@@ -70,17 +112,21 @@ __global__ void k_reconstruct_adj(Geo g, const double2* __restrict__ lu, const d
 // and ny-1 of wall_out, a spectral field whose interior rows the caller fills
 // later); and in hv_old / hg_old the cotangents of the previous stage's terms.
 __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update_adj(
-    Geo g, EigTables t, StageCoef sc, int last, const double* __restrict__ vn_bar_a,
+    Geo g, EigTables t, StageCoef sc, MeanFlowAdj mf, int last, const double* __restrict__ vn_bar_a,
     const double* __restrict__ vn_bar_b, const double* __restrict__ omn_bar, double* __restrict__ hv_old,
     double* __restrict__ hg_old, double* __restrict__ X1_bar, double* __restrict__ T0_bar,
     double* __restrict__ T1_bar, double* __restrict__ vt_bar, double* __restrict__ omt_bar,
     double* __restrict__ wall_out) {
   pdl();
+  if ((int)blockIdx.x < mf.blocks) {
+    mean_flow_adj_block(g, mf, blockIdx.x);
+    return;
+  }
   __shared__ double red[kEigParts][4][kEigCols];
   const int N = 2 * g.nk;
   const int lane = threadIdx.x % kEigCols;
   const int part = threadIdx.x / kEigCols;
-  const int c = blockIdx.x * kEigCols + lane;
+  const int c = (blockIdx.x - mf.blocks) * kEigCols + lane;
   const bool active = c < N;
   const int n = g.ny - 2;
   const int j0 = (n * part) / kEigParts, j1 = (n * (part + 1)) / kEigParts;
@@ -174,43 +220,6 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update_adj(
     }
     wall_out[c] = a0;
     wall_out[(size_t)(g.ny - 1) * N + c] = aN;
-  }
-}
-
-// 7'. Transpose of the (0,0) mean-flow update of stage s: x00_bar <- LR^T
-// ubar, f_bar = Linv^T ubar; conv_bar (this stage) -= dt_e gamma f_bar,
-// conv_bar_prev -= dt_e xi f_bar (null for the first stage). lrT / liT are the
-// stage's transposed matrices (2 Ny x 2 Ny, row-major). One warp per row of
-// the transposed product.
-__global__ void __launch_bounds__(32 * kMeanFlowRows) k_mean_flow_adj(
-    Geo g, const double* __restrict__ lrT, const double* __restrict__ liT, const double2* __restrict__ ubar,
-    double dt_gamma, double dt_xi, double2* __restrict__ x00_out, double2* __restrict__ conv_bar,
-    double2* __restrict__ conv_bar_prev) {
-  pdl();
-  const int n2 = 2 * g.ny;
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * kMeanFlowRows + (threadIdx.x >> 5);
-  if (i >= n2) return;
-  const double* lr = lrT + (size_t)i * n2;
-  const double* li = liT + (size_t)i * n2;
-  double ax = 0.0, ay = 0.0, fx = 0.0, fy = 0.0;
-  for (int j = lane; j < n2; j += 32) {
-    const double2 b = ubar[j];
-    ax += lr[j] * b.x;
-    ay += lr[j] * b.y;
-    fx += li[j] * b.x;
-    fy += li[j] * b.y;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ax += __shfl_down_sync(0xffffffffu, ax, o);
-    ay += __shfl_down_sync(0xffffffffu, ay, o);
-    fx += __shfl_down_sync(0xffffffffu, fx, o);
-    fy += __shfl_down_sync(0xffffffffu, fy, o);
-  }
-  if (lane == 0) {
-    x00_out[i] = make_double2(ax, ay);
-    conv_bar[i] = csub(conv_bar[i], make_double2(dt_gamma * fx, dt_gamma * fy));
-    if (conv_bar_prev) conv_bar_prev[i] = csub(conv_bar_prev[i], make_double2(dt_xi * fx, dt_xi * fy));
   }
 }
 

@@ -6,11 +6,12 @@
 //      k_linear_terms            (linearised equations)
 //   3  k_omega          omega_y of the current state
 //   4  k_dgemm          eigenbasis transforms (V^-1 D q, V^-1 [H1, h_g, v, omega])
-//   5  k_eigen_update   diagonal solves + influence-matrix correction
-//   6  k_mean_flow      (0,0) mean-flow block system
-//   7  k_dgemm          back-transform: v, dv/dy, omega_y
-//   8  k_reconstruct    u, w from continuity, walls
-// and, with constant mass flux, 3 more launches and one copy per step.
+//   5  k_eigen_update   diagonal solves + influence-matrix correction, and the
+//                       (0,0) mean-flow block system in blocks of its own
+//   6  k_dgemm          back-transform: v, dv/dy, omega_y
+//   7  k_reconstruct    u, w from continuity, walls
+// and, with constant mass flux, 2 more launches per step. (k_dgemm: k_parity or
+// another of the product kernels.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1024,30 +1025,27 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
     const double* omt = p->om_valid ? p->omnt : p->T + 3 * E;
     if (p->ev_valid) std::swap(p->vnt, p->vnt_alt);
     if (p->om_valid) std::swap(p->omnt, p->omnt_alt);
-    const int blocks = (N + kEigCols - 1) / kEigCols, rpp = eigen_update_rpp(ny);
-    const size_t sm = eigen_update_smem(ny);
-    if (split_in)
-      run(k_eigen_update<float>, blocks, kEigCols * kEigParts, sm, s, g, t, sc,
-          reinterpret_cast<const float*>(p->X1), reinterpret_cast<const float*>(p->T),
-          reinterpret_cast<const float*>(p->T + E), vt, omt, (const double*)v, reinterpret_cast<float*>(p->hv_old),
-          reinterpret_cast<float*>(p->hg_old), p->vnt, p->omnt, rpp);
-    else
-      run(k_eigen_update<double>, blocks, kEigCols * kEigParts, sm, s, g, t, sc, p->X1, p->T, p->T + E, vt, omt,
-          (const double*)v, p->hv_old, p->hg_old, p->vnt, p->omnt, rpp);
-    JSD_LAUNCHED("k_eigen_update");
-  }
-  {
     const size_t n2 = 2 * (size_t)ny;
-    const double* lns = p->lhs_inv_ns + (size_t)st * n2 * n2;
-    const double2* conv = p->conv + (size_t)st * 2 * gp.ny;
-    const double2* conv_old = st == 0 ? nullptr : p->conv + (size_t)(st - 1) * 2 * gp.ny;
     const double dte = p->desc.dt_explicit;
-    // per-run matrices: lr / lns point at run 0's stage-st matrices, the kernel offsets by run
-    const double* lr = p->lr_ns + (size_t)st * n2 * n2;
-    const dim3 grid((unsigned)((n2 + kMeanFlowRows - 1) / kMeanFlowRows), (unsigned)g.nb);
-    run(k_mean_flow_rows, grid, 32 * kMeanFlowRows, sizeof(double2) * 2 * n2, s, g, lr, lns, u, w, conv, conv_old,
-        dpdx, p->dpdx_scale, dte * kGamma[st], dte * kXi[st], p->uw00);
-    JSD_LAUNCHED("k_mean_flow_rows");
+    // per-run matrices: lr / li point at run 0's stage-st matrices, the kernel offsets by run
+    MeanFlow mf{p->lr_ns + (size_t)st * n2 * n2, p->lhs_inv_ns + (size_t)st * n2 * n2, u, w,
+                p->conv + (size_t)st * 2 * gp.ny, st == 0 ? nullptr : p->conv + (size_t)(st - 1) * 2 * gp.ny, dpdx,
+                p->dpdx_scale, dte * kGamma[st], dte * kXi[st], p->uw00, 0};
+    auto launch = [&](auto ti, auto parts) {
+      using TI = decltype(ti);
+      constexpr int PARTS = decltype(parts)::value;
+      mf.blocks = ((int)n2 + PARTS - 1) / PARTS;
+      const int blocks = mf.blocks * g.nb + (N + kEigCols - 1) / kEigCols;
+      run(k_eigen_update<TI, PARTS>, blocks, kEigCols * PARTS, eigen_update_smem(ny, PARTS), s, g, t, sc, mf,
+          reinterpret_cast<const TI*>(p->X1), reinterpret_cast<const TI*>(p->T), reinterpret_cast<const TI*>(p->T + E),
+          vt, omt, (const double*)v, reinterpret_cast<TI*>(p->hv_old), reinterpret_cast<TI*>(p->hg_old), p->vnt,
+          p->omnt, eigen_update_rpp(ny, PARTS));
+    };
+    using Four = std::integral_constant<int, kEigParts>;
+    if (split_in) launch(float{}, Four{});
+    else if (p->mixed) launch(double{}, Four{});
+    else launch(double{}, std::integral_constant<int, kEigParts64>{});
+    JSD_LAUNCHED("k_eigen_update");
   }
   {
     GemmBatch b = gemm_batch(p);
@@ -1067,15 +1065,13 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
 
 int mass_flux(jsd_plan* p, double2* state, double* dpdx, cudaStream_t s) {
   const Geo& g = p->g;
-  const size_t fs = (size_t)g.ny * g.nk;
   run(k_plane_sums_sliced, dim3(g.ny, kSumSlices), 256, 0, s, g, state, 1, 1, p->partial);
   JSD_LAUNCHED("k_plane_sums_sliced");
-  run(k_mass_flux_scalar_sliced, 1, 32, 0, s, g.ny, p->yw, p->partial, g.c_inv, p->desc.flow_rate_target,
-      p->desc.dt_explicit, dpdx, p->scal);
-  JSD_LAUNCHED("k_mass_flux_scalar_sliced");
-  run(k_roundtrip_shift, grid_for(fs, 256), 256, 0, s, g, state, p->scal, p->tmp);
-  JSD_LAUNCHED("k_roundtrip_shift");
-  JSD_CUDA(cudaMemcpyAsync(state, p->tmp, fs * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+  const size_t quads = (size_t)g.ny * (g.kx_max + 1) * (g.kz_max + 1);
+  // (few blocks: each sums the plane sums again)
+  run(k_mass_flux, std::min(grid_for(quads, 256), 4 * p->num_sms), 256, 0, s, g, p->yw, p->partial,
+      p->desc.flow_rate_target, p->desc.dt_explicit, dpdx, state);
+  JSD_LAUNCHED("k_mass_flux");
   p->om_valid = false;  // u changed; v (and so V^-1 v, dv/dy) did not
   return 0;
 }
@@ -1111,20 +1107,17 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
     StageCoef sc{kAlpha[st], kBeta[st], kGamma[st], kXi[st], p->desc.dt, p->desc.dt_explicit, p->desc.re_tau,
                  st == 0 ? 1 : 0};
     const int N = 2 * g.nk;
-    run(k_eigen_update_adj, (N + kEigCols - 1) / kEigCols, kEigCols * kEigParts, 0, s, g, t, sc, last ? 1 : 0,
-        p->T + 0 * E, p->T + 1 * E, p->T + 2 * E, p->hv_old, p->hg_old, p->X1, p->T + 3 * E, p->vnt, p->omnt,
-        p->vnt_alt, (double*)p->tmp);
-    JSD_LAUNCHED("k_eigen_update_adj");
-  }
-  // 7'
-  {
+    // 7', in blocks of its own
     const size_t n2 = 2 * (size_t)ny;
     const double dte = p->desc.dt_explicit;
-    const unsigned grid = (unsigned)((n2 + kMeanFlowRows - 1) / kMeanFlowRows);
-    run(k_mean_flow_adj, grid, 32 * kMeanFlowRows, 0, s, g, p->lr_T + (size_t)st * n2 * n2,
-        p->li_T + (size_t)st * n2 * n2, p->adj_ub, dte * kGamma[st], dte * kXi[st], p->adj_x00,
-        p->adj_conv + (size_t)st * n2, st > 0 ? p->adj_conv + (size_t)(st - 1) * n2 : nullptr);
-    JSD_LAUNCHED("k_mean_flow_adj");
+    const MeanFlowAdj mf{p->lr_T + (size_t)st * n2 * n2, p->li_T + (size_t)st * n2 * n2, p->adj_ub, dte * kGamma[st],
+                         dte * kXi[st], p->adj_x00, p->adj_conv + (size_t)st * n2,
+                         st > 0 ? p->adj_conv + (size_t)(st - 1) * n2 : nullptr,
+                         ((int)n2 + kEigParts - 1) / kEigParts};
+    run(k_eigen_update_adj, mf.blocks + (N + kEigCols - 1) / kEigCols, kEigCols * kEigParts, 0, s, g, t, sc, mf,
+        last ? 1 : 0, p->T + 0 * E, p->T + 1 * E, p->T + 2 * E, p->hv_old, p->hg_old, p->X1, p->T + 3 * E, p->vnt,
+        p->omnt, p->vnt_alt, (double*)p->tmp);
+    JSD_LAUNCHED("k_eigen_update_adj");
   }
   // 5': cotangents of q (all rows), H1, h_g, the interior of v and of omega_y
   {
@@ -1147,7 +1140,14 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
   // 1': v_bar += D^T dv_bar
   {
     GemmBatch b = gemm_batch(p);
-    add_entry(b, p->D_T, (const double*)(p->Dfld + fs), (double*)(p->Dfld + 2 * fs), ny, ny);
+    add_entry(b, p->D_T, (const double*)(p->Dfld + fs), (double*)lv, ny, ny);
+    ParityBatch o;
+    bool fold = false;
+    if (parity_batch(p, b, o, fold)) {
+      o.accumulate = 1;
+      return launch_parity(p, o, fold, s);
+    }
+    b.e[0].C = (double*)(p->Dfld + 2 * fs);
     int rc = launch_gemm(p, b, ny, kSiteDfield, s);
     if (rc) return rc;
   }
@@ -1192,10 +1192,9 @@ int set_smem_limits() {
     }
     JSD_CUDA(e);
   }
-  JSD_CUDA(cudaFuncSetAttribute(k_mean_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  JSD_CUDA(cudaFuncSetAttribute(k_mean_flow_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  JSD_CUDA(cudaFuncSetAttribute(k_eigen_update<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  JSD_CUDA(cudaFuncSetAttribute(k_eigen_update<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  JSD_CUDA(cudaFuncSetAttribute(k_eigen_update<double, kEigParts64>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  JSD_CUDA(cudaFuncSetAttribute(k_eigen_update<double, kEigParts>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  JSD_CUDA(cudaFuncSetAttribute(k_eigen_update<float, kEigParts>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   JSD_CUDA(cudaFuncSetAttribute(k_tc05_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
   JSD_CUDA(cudaFuncSetAttribute(k_oz8_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
   cudaError_t err = cudaSuccess;
@@ -1401,19 +1400,8 @@ int jsd_autotune(jsd_plan* plan, void* stream) {
     }
     // eigenbasis sites of mixed plans: the Ozaki int8 kernel against the best DMMA tile
     if (rc == 0 && site != kSiteDfield && plan->oz_ready && plan->mixed) {
-      ParityBatch o;
-      bool fold = false;
-      if (parity_batch(plan, b, o, fold)) {
-        // what kernel 0 of the site runs
-        rc = launch_parity(plan, o, fold, s);
-        if (rc == 0 && cudaEventRecord(e0, s) != cudaSuccess) rc = fail(JSD_ERR_CUDA, "cudaEventRecord");
-        for (int r = 0; r < 5 && rc == 0; ++r) rc = launch_parity(plan, o, fold, s);
-        if (rc == 0 && (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-                        cudaEventElapsedTime(&best, e0, e1) != cudaSuccess))
-          rc = fail(JSD_ERR_CUDA, "autotune timing");
-      }
       plan->eig_ms[site][0] = best / 5.f;
-      if (rc == 0) rc = launch_ozaki(plan, b, s);  // warm-up
+      rc = launch_ozaki(plan, b, s);  // warm-up
       if (rc == 0 && cudaEventRecord(e0, s) != cudaSuccess) rc = fail(JSD_ERR_CUDA, "cudaEventRecord");
       for (int r = 0; r < 5 && rc == 0; ++r) rc = launch_ozaki(plan, b, s);
       float ms = 0.f;
@@ -1606,13 +1594,13 @@ int jsd_launches_per_step(const jsd_plan* plan) {
   const bool linear = plan->desc.linearise && plan->desc.kind != JSD_KIND_NS;
   // steady state: each stage launches dfield (not for the linear terms, which take
   // dv/dy carried from the last stage), nonlinear terms (3 transforms or 1 linear
-  // kernel), 2 GEMMs, eigen update, mean flow and reconstruct; omega_y is carried
-  // too, except after the mass-flux correction (3 launches) changed u
+  // kernel), 2 GEMMs, eigen update (with the mean flow) and reconstruct; omega_y is
+  // carried too, except after the mass-flux correction (2 launches) changed u
   const bool coupling_off = !plan->coupling && plan->desc.kind != JSD_KIND_NS;
   // a source (jsd_set_source) adds k_add_source and k_add_source00 per stage
-  const int per_stage = (linear ? 6 : 9) + (coupling_off ? 1 : 0) + (plan->src_hv ? 2 : 0);
+  const int per_stage = (linear ? 5 : 8) + (coupling_off ? 1 : 0) + (plan->src_hv ? 2 : 0);
   const bool cmf = plan->desc.constant_mass_flux != 0;
-  return 3 * per_stage + (cmf ? 3 + 1 : 0);
+  return 3 * per_stage + (cmf ? 2 + 1 : 0);
 }
 
 }  // extern "C"
@@ -1628,7 +1616,6 @@ namespace {
 struct SymTables {
   bool ok = false;
   int n_even = 0;
-  std::vector<int> order;  // the caller's eigen index of each row
   std::vector<double> D, V, Vinv, lam, sgn, c0, cN, w0, wN;
 };
 
@@ -1644,7 +1631,7 @@ SymTables symmetric_tables(const jsd_desc* d) {
     vmax = std::max(vmax, std::fabs(d->V[i]));
     wmax = std::max(wmax, std::fabs(d->Vinv[i]));
   }
-  std::vector<int>& order = t.order;
+  std::vector<int> order;
   for (int want : {1, -1})
     for (int j = 0; j < n; ++j)
       if (d->sgn[j] == want) order.push_back(j);
@@ -1778,11 +1765,11 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     return fail(JSD_ERR_ARG, "FFT length must factor into 2, 3, 5, 7");
   }
   const int ny = d->ny, ni = ny - 2;
-  // Mixed plans under flow control keep the caller's tables and whole
-  // operators: there the products' round-off decides FP32 roundings, and dP/dx,
-  // a difference of flow rates over dt, shows them (1e-8 of it where it is small).
-  const SymTables sym = p->mixed && d->constant_mass_flux ? SymTables() : symmetric_tables(d);
-  const jsd_desc* given = d;
+  // Mixed plans keep the caller's tables and whole operators: the products'
+  // round-off decides FP32 roundings downstream, so another product order moves
+  // their results by a part of their own error (dP/dx, a small difference of flow
+  // rates over dt, by 1e-8 of itself).
+  const SymTables sym = p->mixed ? SymTables() : symmetric_tables(d);
   jsd_desc own = *d;  // the caller's description with the plan's own tables
   if (sym.ok) {
     own.D = sym.D.data();
@@ -1865,7 +1852,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     std::vector<float> hi((size_t)ny * p->lda, 0.f), lo((size_t)ny * p->lda, 0.f);
     for (int r = 0; r < ny; ++r)
       for (int c = 0; c < ny; ++c) {
-        const double x = given->D[(size_t)r * ny + c];
+        const double x = d->D[(size_t)r * ny + c];
         const float h = tf32_round((float)x);
         hi[(size_t)r * p->lda + c] = h;
         lo[(size_t)r * p->lda + c] = tf32_round((float)(x - (double)h));
@@ -1873,19 +1860,8 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     JSD_TRY(upload(p, &p->Dhi, hi.data(), hi.size()));
     JSD_TRY(upload(p, &p->Dlo, lo.data(), lo.size()));
     // V^-1 D and V^-1 split the same way (eigenbasis-in products of the
-    // FP32-accurate nonlinear terms). These parts, like D's, come from the
-    // caller's own tables: the split's last bit would move with their round-off
-    std::vector<double> gVinv((size_t)ni * ni), gVinvD((size_t)ni * ny);
-    for (int i = 0; i < ni; ++i) {
-      const double* row = given->Vinv + (size_t)(sym.ok ? sym.order[i] : i) * ni;
-      std::copy(row, row + ni, gVinv.begin() + (size_t)i * ni);
-      for (int c = 0; c < ny; ++c) {
-        long double acc = 0;
-        for (int j = 0; j < ni; ++j) acc += (long double)row[j] * given->D[(size_t)(j + 1) * ny + c];
-        gVinvD[(size_t)i * ny + c] = (double)acc;
-      }
-    }
-    const double* eiA[2] = {gVinvD.data(), gVinv.data()};
+    // FP32-accurate nonlinear terms)
+    const double* eiA[2] = {VinvD.data(), d->Vinv};
     const int eiK[2] = {ny, ni};
     for (int k = 0; k < 2; ++k) {
       std::vector<float> eh((size_t)ni * p->lda, 0.f), el((size_t)ni * p->lda, 0.f);
@@ -1908,7 +1884,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
     if (ny <= kTcM + 1) {
       p->tc_rows = ny;
       std::vector<float> ahi, alo;
-      tc05_pack_a(given->D, ny, ny, ny, tf32_round, ahi, alo);
+      tc05_pack_a(d->D, ny, ny, ny, tf32_round, ahi, alo);
       JSD_TRY(upload(p, &p->tc_ahi, ahi.data(), ahi.size()));
       JSD_TRY(upload(p, &p->tc_alo, alo.data(), alo.size()));
       for (int k = 0; k < 2; ++k) {
@@ -1918,7 +1894,7 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
       }
       if (ny > kTcM) {
         std::vector<double> xr(kTcKp, 0.0);
-        for (int c = 0; c < ny; ++c) xr[c] = given->D[(size_t)kTcM * ny + c];
+        for (int c = 0; c < ny; ++c) xr[c] = d->D[(size_t)kTcM * ny + c];
         JSD_TRY(upload(p, &p->tc_xrow, xr.data(), xr.size()));
       }
       // the tcgen05 kernel is the default (58 us per call against 86 us for
@@ -2144,7 +2120,7 @@ int jsd_correct_mass_flux(jsd_plan* plan, void* state, double* dpdx, void* strea
   if (plan->g.nb > 1) return fail(JSD_ERR_ARG, "single-run entry point called on a batch plan (see jsd_energy_runs)");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const ProgrammaticLaunches pl(plan, s);
-  double* dp = dpdx ? dpdx : plan->scal + 1;  // a scratch slot when the caller keeps no pressure gradient
+  double* dp = dpdx ? dpdx : plan->scal;  // a scratch slot when the caller keeps no pressure gradient
   plan->ev_valid = plan->om_valid = plan->dv_valid = false;
   return mass_flux(plan, static_cast<double2*>(state), dp, s);
 }

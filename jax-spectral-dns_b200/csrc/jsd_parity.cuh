@@ -53,6 +53,7 @@ struct ParityBatch {
   int N;       // columns = row stride of B and C
   int unfold;  // outputs on the points (else: rows of half 0, then of half 1)
   int rows;    // rows of a tile buffer (parity_rows)
+  int accumulate;  // C += A B (unfolded outputs only)
 };
 
 // row tiles of 8 that hold M rows, one row beyond them left to the dot products
@@ -374,11 +375,15 @@ __global__ void __launch_bounds__(64 * W, ParityCfg<W, TM>::MIN_BLOCKS) k_parity
 #pragma unroll
             for (int q = 0; q < 2; ++q) o[q] = xc[((((1 - h) * TM + i) * HJ + j) * 2 + q) * 32];
             const double* m = acc[i][h * HJ + j];
+            double2 up = make_double2(m[0] + o[0], m[1] + o[1]);
+            double2 dn = h ? make_double2(o[0] - m[0], o[1] - m[1]) : make_double2(m[0] - o[0], m[1] - o[1]);
             if (full || col + 8 * j < N) {
-              if (r < mout - pairs) *reinterpret_cast<double2*>(Cu + 8 * j) = make_double2(m[0] + o[0], m[1] + o[1]);
-              if (r < pairs)
-                *reinterpret_cast<double2*>(Cd + 8 * j) =
-                    h ? make_double2(o[0] - m[0], o[1] - m[1]) : make_double2(m[0] - o[0], m[1] - o[1]);
+              if (batch.accumulate) {
+                if (r < mout - pairs) up = cadd(up, *reinterpret_cast<double2*>(Cu + 8 * j));
+                if (r < pairs) dn = cadd(dn, *reinterpret_cast<double2*>(Cd + 8 * j));
+              }
+              if (r < mout - pairs) *reinterpret_cast<double2*>(Cu + 8 * j) = up;
+              if (r < pairs) *reinterpret_cast<double2*>(Cd + 8 * j) = dn;
             }
           }
         }
@@ -397,8 +402,10 @@ __global__ void __launch_bounds__(64 * W, ParityCfg<W, TM>::MIN_BLOCKS) k_parity
           S += xrow[q * kParN + lane];
           T += xrow[(2 * W + q) * kParN + lane];
         }
-        C[(size_t)(8 * RT) * N + lane] = S + T;
-        if (pairs > 8 * RT) C[(size_t)(mout - 1 - 8 * RT) * N + lane] = S - T;
+        double* Cu = C + (size_t)(8 * RT) * N + lane;
+        double* Cd = C + (size_t)(mout - 1 - 8 * RT) * N + lane;
+        *Cu = S + T + (batch.accumulate ? *Cu : 0.0);
+        if (pairs > 8 * RT) *Cd = S - T + (batch.accumulate ? *Cd : 0.0);
       }
     }
     ei = ein;

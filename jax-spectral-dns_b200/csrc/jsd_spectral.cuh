@@ -573,6 +573,65 @@ __global__ void k_omega(Geo g, const double2* __restrict__ u, const double2* __r
 }
 
 // ---------------------------------------------------------------------------
+// (0,0) mean flow: the reference's 2Ny x 2Ny system for (U00, W00)
+// (navier_stokes.py:1417-1504) with its own matrices:
+//   x_new = Linv_ns (R_ns x + dt_e gamma N + dt_e xi N_old),
+//   N = [-conv00_x - dpdx * scale, -conv00_z]
+// (g.ny = Chebyshev points, g.nb runs; conv entries per plane, matrices and
+// uw00 per run; conv_old == nullptr means zero.)
+// ---------------------------------------------------------------------------
+// Row-parallel form of the same update with LR = Linv_ns R_ns precomputed per
+// stage: x_new = LR x + Linv_ns (dt_e gamma N + dt_e xi N_old). One warp per
+// output row; every block first builds x and the forcing f = dt_e gamma N +
+// dt_e xi N_old of its run in shared memory (4 Ny entries). It depends on
+// neither the eigenbasis products nor the update, so its blocks lead the grid
+// of k_eigen_update (a launch of its own took 9 us between two kernels).
+struct MeanFlow {
+  const double *lr, *li;            // run 0's stage matrices (3 (2 Ny)^2 apart per run)
+  const double2 *u, *w;             // the state's fields
+  const double2 *conv, *conv_old;   // conv_old: null for the first stage
+  const double* dpdx;
+  double dpdx_scale, dt_gamma, dt_xi;
+  double2* uw00;
+  int blocks;                       // blocks per run; rows per block = warps per block
+};
+
+__device__ __forceinline__ void mean_flow_block(const Geo& g, const MeanFlow& m, int block, double2* msm) {
+  const int n = g.ny, n2 = 2 * g.ny;
+  const int run = block / m.blocks, nb = g.nb;
+  const double* lr_ns = m.lr + (size_t)run * 3 * n2 * n2;
+  const double* lhs_inv_ns = m.li + (size_t)run * 3 * n2 * n2;
+  double2* xv = msm;      // (U00, W00) of the run
+  double2* fv = xv + n2;  // forcing
+  const double dp = m.dpdx ? m.dpdx[0] * m.dpdx_scale : 0.0;
+  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+    const int ci = (i < n) ? i * nb + run : n * nb + (i - n) * nb + run;
+    xv[i] = (i < n) ? m.u[sidx(g, i * nb + run, 0, 0)] : m.w[sidx(g, (i - n) * nb + run, 0, 0)];
+    const double src = (i < n) ? -dp : 0.0;
+    const double2 nn = make_double2(-m.conv[ci].x + src, -m.conv[ci].y);
+    const double2 no =
+        m.conv_old ? make_double2(-m.conv_old[ci].x + src, -m.conv_old[ci].y) : make_double2(src, 0.0);
+    fv[i] = cadd(cscale(nn, m.dt_gamma), cscale(no, m.dt_xi));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int i = (block - run * m.blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= n2) return;
+  const double* lr = lr_ns + (size_t)i * n2;
+  const double* li = lhs_inv_ns + (size_t)i * n2;
+  double ax = 0.0, ay = 0.0;
+  for (int j = lane; j < n2; j += 32) {
+    ax += lr[j] * xv[j].x + li[j] * fv[j].x;
+    ay += lr[j] * xv[j].y + li[j] * fv[j].y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    ax += __shfl_down_sync(0xffffffffu, ax, o);
+    ay += __shfl_down_sync(0xffffffffu, ay, o);
+  }
+  if (lane == 0) m.uw00[(size_t)run * n2 + i] = make_double2(ax, ay);
+}
+
+// ---------------------------------------------------------------------------
 // Per-column eigenbasis update of the Helmholtz / Poisson / influence-matrix
 // solve (navier_stokes.py:1291-1414). In the eigenbasis D2_int = V diag(lam) V^-1
 // every per-wavenumber operator is diagonal; L_j = lam_j - k^2:
@@ -602,34 +661,53 @@ struct StageCoef {
 };
 
 constexpr int kEigCols = 32;    // columns per block (one warp-wide row segment)
-constexpr int kEigParts = 4;    // warps per block, each walking a quarter of the eigen rows
+constexpr int kEigParts = 4;    // warps per block of the mixed form and of the adjoint, each a quarter of the eigen rows
 constexpr int kEigBatch = 4;    // rows whose loads are issued together (loads in flight per thread: 7 x batch)
 
-// Rows of a block's part: j1 - j0 <= ceil((Ny - 2) / kEigParts). The first
-// pass keeps v_p~ of its rows in shared memory for the second (rpp rows per
-// part, dynamic shared memory of eigen_update_smem bytes).
-inline int eigen_update_rpp(int ny) { return (ny - 2 + kEigParts - 1) / kEigParts; }
-inline size_t eigen_update_smem(int ny) { return sizeof(double) * kEigParts * eigen_update_rpp(ny) * kEigCols; }
+// The FP64 form runs eight parts: half as long a chain of rows per thread, which
+// is the whole time of a small box (9 x 65 x 5 modes 8.8 us with the mean flow,
+// 13.5 + 6 us with four parts and a launch of its own; 129 x 129 x 129, bound by
+// HBM at 57 us, 73 against 70 + 9). The mixed form keeps four: another grouping
+// of the influence sums moves its rounding.
+constexpr int kEigParts64 = 8;
+
+// Rows of a block's part: j1 - j0 <= ceil((Ny - 2) / parts). The first pass
+// keeps v_p~ (and, with eight parts, 1 / (H L)) of its rows in shared memory for
+// the second (rpp rows per part, dynamic shared memory of eigen_update_smem bytes).
+inline int eigen_update_rpp(int ny, int parts) { return (ny - 2 + parts - 1) / parts; }
+inline size_t eigen_update_smem(int ny, int parts) {
+  const size_t rows =
+      sizeof(double) * (parts > kEigParts ? 2 : 1) * parts * eigen_update_rpp(ny, parts) * kEigCols;
+  const size_t mean = sizeof(double2) * 4 * (size_t)ny;
+  return rows > mean ? rows : mean;
+}
 
 // TI: storage of the nonlinear terms (X1, H1~, h_g~ and the previous stage's
 // h_v~, h_g~): double, or float where they come out of FP32 transforms and
-// products (the mixed form)
-template <typename TI>
-__global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update(
-    Geo g, EigTables t, StageCoef sc, const TI* __restrict__ X1, const TI* __restrict__ H1t,
+// products (the mixed form). The first mf.blocks * g.nb blocks are the mean flow's.
+template <typename TI, int PARTS>
+__global__ void __launch_bounds__(kEigCols * PARTS, PARTS > kEigParts ? 2 : 4) k_eigen_update(
+    Geo g, EigTables t, StageCoef sc, MeanFlow mf, const TI* __restrict__ X1, const TI* __restrict__ H1t,
     const TI* __restrict__ hgt, const double* __restrict__ vt, const double* __restrict__ omt,
     const double* __restrict__ vfield, TI* __restrict__ hv_old, TI* __restrict__ hg_old,
     double* __restrict__ vnt, double* __restrict__ omnt, int rpp) {
   pdl();
-  __shared__ double red[kEigParts][6][kEigCols];
-  extern __shared__ double vps_all[];
+  constexpr bool KEEP = PARTS > kEigParts;
+  __shared__ double red[PARTS][6][kEigCols];
+  extern __shared__ __align__(16) double vps_all[];
+  const int lead = mf.blocks * g.nb;
+  if ((int)blockIdx.x < lead) {
+    mean_flow_block(g, mf, blockIdx.x, reinterpret_cast<double2*>(vps_all));
+    return;
+  }
   const int N = 2 * g.nk * g.nb;  // columns: real and imaginary parts of every mode of every run
   const int lane = threadIdx.x % kEigCols;
   const int part = threadIdx.x / kEigCols;
-  const int c = blockIdx.x * kEigCols + lane;
+  const int c = (blockIdx.x - lead) * kEigCols + lane;
   const bool active = c < N;
   const int n = g.ny - 2;
-  const int j0 = (n * part) / kEigParts, j1 = (n * (part + 1)) / kEigParts;
+  const int j0 = (n * part) / PARTS, j1 = (n * (part + 1)) / PARTS;
+  double* ihls = vps_all + (size_t)(PARTS + part) * rpp * kEigCols + lane;
   double* vps = vps_all + (size_t)part * rpp * kEigCols + lane;  // v_p~ of row j at vps[(j - j0) * kEigCols]
   double k2 = 0.0, v0 = 0.0, vN = 0.0, re = sc.re;
   if (active) {
@@ -692,6 +770,7 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update(
         d0b += w0 * sg * va;
         dNb += wN * sg * va;
         vps[(j - j0) * kEigCols] = vp;
+        if (KEEP) ihls[(j - j0) * kEigCols] = ihl;
         hv_old[o] = (TI)hv;
         omnt[o] = (R * om[b] + sc.dt_e * (sc.gamma * (double)hg[b] + sc.xi * (double)hgo[b])) * ih;
         hg_old[o] = hg[b];
@@ -711,7 +790,7 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update(
   for (int q = 0; q < 6; ++q) {
     double acc = 0.0;
 #pragma unroll
-    for (int pp = 0; pp < kEigParts; ++pp) acc += red[pp][q][lane];
+    for (int pp = 0; pp < PARTS; ++pp) acc += red[pp][q][lane];
     sum[q] = acc;
   }
   const double det = sum[2] * sum[5] - sum[4] * sum[3];
@@ -719,124 +798,17 @@ __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update(
   const double a = (sum[5] * ra - sum[4] * rb) / det;
   const double b = (-sum[3] * ra + sum[2] * rb) / det;
   for (int j = j0; j < j1; ++j) {
-    const double L = t.lam[j] - k2;
-    const double H = 1.0 - br * L;
-    const double va = br * t.c0[j] * (1.0 / (H * L));
+    double ihl;
+    if (KEEP) {
+      ihl = ihls[(j - j0) * kEigCols];
+    } else {
+      const double L = t.lam[j] - k2;
+      const double H = 1.0 - br * L;
+      ihl = 1.0 / (H * L);
+    }
+    const double va = br * t.c0[j] * ihl;
     vnt[(size_t)j * N + c] = vps[(j - j0) * kEigCols] + (a + b * t.sgn[j]) * va;
   }
-}
-
-// ---------------------------------------------------------------------------
-// (0,0) mean flow: the reference's 2Ny x 2Ny system for (U00, W00)
-// (navier_stokes.py:1417-1504) with its own matrices:
-//   x_new = Linv_ns (R_ns x + dt_e gamma N + dt_e xi N_old),
-//   N = [-conv00_x - dpdx * scale, -conv00_z]
-// One block per run (g.ny = Chebyshev points, g.nb runs; conv entries per plane,
-// matrices and uw00 per run). conv_old == nullptr means zero.
-// ---------------------------------------------------------------------------
-constexpr int kMeanFlowThreads = 1024;
-
-__global__ void __launch_bounds__(kMeanFlowThreads) k_mean_flow(
-    Geo g, const double* __restrict__ rhs_ns, const double* __restrict__ lhs_inv_ns, const double2* __restrict__ u,
-    const double2* __restrict__ w, const double2* __restrict__ conv, const double2* __restrict__ conv_old,
-    const double* __restrict__ dpdx, double dpdx_scale, double dt_gamma, double dt_xi, double2* __restrict__ uw00) {
-  pdl();
-  extern __shared__ __align__(16) double2 msm[];
-  const int n = g.ny, n2 = 2 * g.ny;
-  // block = run of a batch: its matrices, its planes (y * nb + run) and conv entries
-  const int run = blockIdx.x, nb = g.nb;
-  rhs_ns += (size_t)run * 3 * n2 * n2;
-  lhs_inv_ns += (size_t)run * 3 * n2 * n2;
-  uw00 += (size_t)run * n2;
-  double2* xv = msm;       // current (U00, W00)
-  double2* rv = xv + n2;   // right-hand side
-  const double dp = dpdx ? dpdx[0] * dpdx_scale : 0.0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  auto cidx = [&](int i) { return (i < n) ? i * nb + run : n * nb + (i - n) * nb + run; };
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-    xv[i] = (i < n) ? u[sidx(g, i * nb + run, 0, 0)] : w[sidx(g, (i - n) * nb + run, 0, 0)];
-  }
-  __syncthreads();
-  // one warp per row, lanes along the row (coalesced)
-  for (int i = warp; i < n2; i += nwarps) {
-    const double* row = rhs_ns + (size_t)i * n2;
-    double ax = 0.0, ay = 0.0;
-    for (int j = lane; j < n2; j += 32) {
-      ax += xv[j].x * row[j];
-      ay += xv[j].y * row[j];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      ax += __shfl_down_sync(0xffffffffu, ax, o);
-      ay += __shfl_down_sync(0xffffffffu, ay, o);
-    }
-    if (lane == 0) {
-      const double src = (i < n) ? -dp : 0.0;
-      const double2 nn = make_double2(-conv[cidx(i)].x + src, -conv[cidx(i)].y);
-      const double2 no =
-          conv_old ? make_double2(-conv_old[cidx(i)].x + src, -conv_old[cidx(i)].y) : make_double2(src, 0.0);
-      rv[i] = cadd(cadd(make_double2(ax, ay), cscale(nn, dt_gamma)), cscale(no, dt_xi));
-    }
-  }
-  __syncthreads();
-  for (int i = warp; i < n2; i += nwarps) {
-    const double* row = lhs_inv_ns + (size_t)i * n2;
-    double ax = 0.0, ay = 0.0;
-    for (int j = lane; j < n2; j += 32) {
-      ax += rv[j].x * row[j];
-      ay += rv[j].y * row[j];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      ax += __shfl_down_sync(0xffffffffu, ax, o);
-      ay += __shfl_down_sync(0xffffffffu, ay, o);
-    }
-    if (lane == 0) uw00[i] = make_double2(ax, ay);
-  }
-}
-
-// Row-parallel form of the same update with LR = Linv_ns R_ns precomputed per
-// stage: x_new = LR x + Linv_ns (dt_e gamma N + dt_e xi N_old). Grid (row
-// blocks, runs), one warp per output row; every block first builds x and the
-// forcing f = dt_e gamma N + dt_e xi N_old of its run in shared memory.
-constexpr int kMeanFlowRows = 8;  // rows (warps) per block
-
-__global__ void __launch_bounds__(32 * kMeanFlowRows) k_mean_flow_rows(
-    Geo g, const double* __restrict__ lr_ns, const double* __restrict__ lhs_inv_ns, const double2* __restrict__ u,
-    const double2* __restrict__ w, const double2* __restrict__ conv, const double2* __restrict__ conv_old,
-    const double* __restrict__ dpdx, double dpdx_scale, double dt_gamma, double dt_xi, double2* __restrict__ uw00) {
-  pdl();
-  extern __shared__ __align__(16) double2 msm[];
-  const int n = g.ny, n2 = 2 * g.ny;
-  const int run = blockIdx.y, nb = g.nb;
-  lr_ns += (size_t)run * 3 * n2 * n2;
-  lhs_inv_ns += (size_t)run * 3 * n2 * n2;
-  uw00 += (size_t)run * n2;
-  double2* xv = msm;      // (U00, W00) of the run
-  double2* fv = xv + n2;  // forcing
-  const double dp = dpdx ? dpdx[0] * dpdx_scale : 0.0;
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-    const int ci = (i < n) ? i * nb + run : n * nb + (i - n) * nb + run;
-    xv[i] = (i < n) ? u[sidx(g, i * nb + run, 0, 0)] : w[sidx(g, (i - n) * nb + run, 0, 0)];
-    const double src = (i < n) ? -dp : 0.0;
-    const double2 nn = make_double2(-conv[ci].x + src, -conv[ci].y);
-    const double2 no = conv_old ? make_double2(-conv_old[ci].x + src, -conv_old[ci].y) : make_double2(src, 0.0);
-    fv[i] = cadd(cscale(nn, dt_gamma), cscale(no, dt_xi));
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * kMeanFlowRows + (threadIdx.x >> 5);
-  if (i >= n2) return;
-  const double* lr = lr_ns + (size_t)i * n2;
-  const double* li = lhs_inv_ns + (size_t)i * n2;
-  double ax = 0.0, ay = 0.0;
-  for (int j = lane; j < n2; j += 32) {
-    ax += lr[j] * xv[j].x + li[j] * fv[j].x;
-    ay += lr[j] * xv[j].y + li[j] * fv[j].y;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ax += __shfl_down_sync(0xffffffffu, ax, o);
-    ay += __shfl_down_sync(0xffffffffu, ay, o);
-  }
-  if (lane == 0) uw00[i] = make_double2(ax, ay);
 }
 
 // u, w from continuity and omega_y (rk_not_00, navier_stokes.py:1506-1527);
@@ -991,65 +963,54 @@ __global__ void k_weighted_total_runs_sliced(int ny, int nb, const double* __res
   if (threadIdx.x == 0) out[run] = scale * a;
 }
 
-// mass-flux scalar from sliced partial sums of Re u, one warp
-__global__ void k_mass_flux_scalar_sliced(int ny, const double* __restrict__ weights,
-                                          const double* __restrict__ partial, double c_inv, double q0, double dt_e,
-                                          double* __restrict__ dpdx, double* __restrict__ qdiff) {
-  pdl();
-  const double a = weighted_slices(ny, 1, 0, weights, partial);
-  if (threadIdx.x == 0) {
-    const double d = c_inv * a - q0;
-    dpdx[0] = dpdx[0] + d / dt_e;
-    qdiff[0] = d;
-  }
-}
-
-// Per-run totals of a batch: out[run] = scale * sum_y w_y partial[y * nb + run]
-// (partial per plane from k_plane_sums).
-__global__ void k_weighted_total_runs(int ny, int nb, const double* __restrict__ weights,
-                                      const double* __restrict__ partial, double scale, double* __restrict__ out) {
-  pdl();
-  const int run = blockIdx.x * blockDim.x + threadIdx.x;
-  if (run >= nb) return;
-  double acc = 0.0;
-  for (int y = 0; y < ny; ++y) acc += weights[y] * partial[(size_t)y * nb + run];
-  out[run] = scale * acc;
-}
-
 // Constant mass flux (navier_stokes.py:724-805, 1205-1214): with the flow rate
 // Q = c_inv * sum_y w_y sum_k Re u(y, k) (the y-integral of u at x = z = 0),
 //   dPdx += (Q - Q0) / dt_e,   u <- RT(u) + const
 // where the constant is -(Q - Q0) / 2 in physical units (walls included).
-__global__ void k_mass_flux_scalar(int ny, const double* __restrict__ weights, const double* __restrict__ partial,
-                                   double c_inv, double q0, double dt_e, double* __restrict__ dpdx,
-                                   double* __restrict__ qdiff) {
+// partial: the plane sums of Re u (k_plane_sums_sliced); every block sums them in
+// the same order, block 0 updates dPdx. u in place: a thread owns the entries at
+// (+-kx, +-kz), which are all that the round trip of any of them reads.
+__global__ void __launch_bounds__(256) k_mass_flux(Geo g, const double* __restrict__ weights,
+                                                   const double* __restrict__ partial, double q0, double dt_e,
+                                                   double* __restrict__ dpdx, double2* __restrict__ u) {
   pdl();
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double acc = 0.0;
-    for (int y = 0; y < ny; ++y) acc += weights[y] * partial[y];
-    const double q = c_inv * acc;
-    const double d = q - q0;
-    dpdx[0] = dpdx[0] + d / dt_e;
-    qdiff[0] = d;
+  __shared__ double off;
+  if (threadIdx.x < 32) {
+    const double a = weighted_slices(g.ny, 1, 0, weights, partial);
+    if (threadIdx.x == 0) {
+      const double d = g.c_inv * a - q0;
+      off = d;
+      if (blockIdx.x == 0) dpdx[0] = dpdx[0] + d / dt_e;
+    }
   }
-}
-
-__global__ void k_roundtrip_shift(Geo g, const double2* __restrict__ f, const double* __restrict__ qdiff,
-                                  double2* __restrict__ out) {
-  pdl();
-  const size_t total = (size_t)g.ny * g.nk;
-  const double shift = -qdiff[0] * 0.5 / g.c_inv;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int y = (int)(t / g.nk);
-    const int r = (int)(t - (size_t)y * g.nk);
-    const int ix = r / g.mz, iz = r - (r / g.mz) * g.mz;
-    int sx, sz;
-    bool cj;
-    truncation_source(g, ix, iz, sx, sz, cj);
-    double2 s = sym_at(g, f, y, sx, sz);
-    if (cj) s = cconj(s);
-    if (ix == 0 && iz == 0) s.x += shift;
-    out[t] = s;
+  __syncthreads();
+  const double shift = -off * 0.5 / g.c_inv;
+  const int K = g.kx_max, Kz = g.kz_max, nq = (K + 1) * (Kz + 1);
+  const size_t total = (size_t)g.ny * nq;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
+    const int y = (int)(q / nq), r = (int)(q - (size_t)y * nq);
+    const int kx = r / (Kz + 1), kz = r - kx * (Kz + 1);
+    const int xm = mode_pos(-kx, g.mx), zm = mode_pos(-kz, g.mz);
+    const size_t o[4] = {sidx(g, y, kx, kz), sidx(g, y, xm, zm), sidx(g, y, kx, zm), sidx(g, y, xm, kz)};
+    double2 f[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = u[o[i]];
+    // Hermitian parts at (kx, kz) and (kx, -kz); at the opposite mode the conjugate
+    const double2 sp = make_double2(0.5 * (f[0].x + f[1].x), 0.5 * (f[0].y - f[1].y));
+    const double2 sm = make_double2(0.5 * (f[2].x + f[3].x), 0.5 * (f[2].y - f[3].y));
+    const double2 np = make_double2(0.5 * (f[1].x + f[0].x), 0.5 * (f[1].y - f[0].y));
+    const double2 nm = make_double2(0.5 * (f[3].x + f[2].x), 0.5 * (f[3].y - f[2].y));
+    const bool qx = kx == K, qz = kz == Kz;  // the -K slot takes the conjugate of the +K one
+    double2 out[4];
+    out[0] = sp;
+    out[1] = qx ? (qz ? sp : cconj(sm)) : (qz ? cconj(nm) : np);
+    out[2] = qz ? cconj(sp) : sm;
+    out[3] = qx ? cconj(sp) : nm;
+    if (kx == 0 && kz == 0) out[0].x += shift;
+    u[o[0]] = out[0];
+    if (kx && kz) u[o[1]] = out[1];
+    if (kz) u[o[2]] = out[2];
+    if (kx) u[o[3]] = out[3];
   }
 }
 
