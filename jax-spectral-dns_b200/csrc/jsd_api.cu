@@ -1043,7 +1043,7 @@ int stage(jsd_plan* p, double2* state, double* dpdx, int st, int time_step, cuda
     };
     using Four = std::integral_constant<int, kEigParts>;
     if (split_in) launch(float{}, Four{});
-    else if (p->mixed) launch(double{}, Four{});
+    else if (p->mixed || eigen_update_smem(ny, kEigParts64) > kEigSmem64) launch(double{}, Four{});
     else launch(double{}, std::integral_constant<int, kEigParts64>{});
     JSD_LAUNCHED("k_eigen_update");
   }

@@ -670,6 +670,10 @@ constexpr int kEigBatch = 4;    // rows whose loads are issued together (loads i
 // HBM at 57 us, 73 against 70 + 9). The mixed form keeps four: another grouping
 // of the influence sums moves its rounding.
 constexpr int kEigParts64 = 8;
+// ... up to Ny = 202, where two blocks of eight parts (two kept arrays, 512 bytes
+// per row) still share an SM; beyond, four parts with one kept array, which fit
+// up to Ny = 802 (eight would be refused from Ny = 403 on).
+constexpr size_t kEigSmem64 = 100 * 1024;
 
 // Rows of a block's part: j1 - j0 <= ceil((Ny - 2) / parts). The first pass
 // keeps v_p~ (and, with eight parts, 1 / (H L)) of its rows in shared memory for
