@@ -306,13 +306,17 @@ namespace {
 // fields that no longer share the L2 on they lose (129 x 129 x 129, 2.1 M entries:
 // 4706 against 4593), and in a captured graph, whose nodes already follow each
 // other closely, they cost 1 us per node (270 nodes at 33 x 65 x 33: 1892 us
-// against 1630), so both keep plain order.
+// against 1630), so both keep plain order. The mixed form loses much earlier
+// (per step: 17 x 65 x 17 174 against 216 us, 33 x 65 x 33 214 / 221, 49 x 33 x 49
+// 188 / 205, but 49 x 65 x 49 324 / 311, 33 x 97 x 33 277 / 272, 49 x 97 x 49 442 /
+// 402, 97 x 97 x 97 1105 / 1080): its line lies between 79 and 106 thousand entries.
 constexpr size_t kProgrammaticMax = 1u << 20;  // entries per field, all runs
+constexpr size_t kProgrammaticMixed = 80000;
 
 struct ProgrammaticLaunches {
   ProgrammaticLaunches(const jsd_plan* p, cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    g_programmatic = (size_t)p->g.ny * p->g.nk * p->g.nb <= kProgrammaticMax &&
+    g_programmatic = (size_t)p->g.ny * p->g.nk * p->g.nb <= (p->mixed ? kProgrammaticMixed : kProgrammaticMax) &&
                      cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
   }
   ~ProgrammaticLaunches() { g_programmatic = false; }
