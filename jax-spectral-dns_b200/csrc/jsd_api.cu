@@ -912,9 +912,15 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
       const C* tab = p->mixed ? (const C*)p->tsqz32 : (const C*)p->tsqz;
       with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
-        const int per_block = kSqWarps * SqLane<S>::G;
-        run(k_zinv_sq<C, S>, (ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zinv_sq_smem<C, S>(), s, g, tab,
-            src, inter);
+        using Z = ZinvStaged<C, S>;
+        const int per_block = kSqWarps * SqLane<S>::G, blocks = (ny * K1 + per_block - 1) / per_block;
+        if constexpr (Z::EVER)
+          if (Z::ALWAYS || fs >= kStagedMin) {
+            run(k_zinv_staged<C, S>, blocks, kSqWarps * 32, Z::smem(g), s, g, tab, src, inter);
+            return;
+          }
+        if constexpr (!Z::ALWAYS)
+          run(k_zinv_sq<C, S>, blocks, kSqWarps * 32, zinv_sq_smem<C, S>(), s, g, tab, src, inter);
       });
       JSD_LAUNCHED("k_zinv_sq");
     } else {
@@ -1209,9 +1215,9 @@ int set_smem_limits() {
   for (int sd : kSquareSides) {
     with_square_side<double2>(sd, [&](auto side) {
       constexpr int S = decltype(side)::value;
-      for (const void* fn : {(const void*)k_zinv_sq<double2, S>, (const void*)k_zfwd_sq<double2, S>,
-                             (const void*)k_xmid_park<XLineLanes<S>>})
-        limit(fn);
+      for (const void* fn : {(const void*)k_zfwd_sq<double2, S>, (const void*)k_xmid_park<XLineLanes<S>>}) limit(fn);
+      if constexpr (ZinvStaged<double2, S>::EVER) limit((const void*)k_zinv_staged<double2, S>);
+      if constexpr (!ZinvStaged<double2, S>::ALWAYS) limit((const void*)k_zinv_sq<double2, S>);
       if constexpr (S <= 7) limit((const void*)k_xmid_dual_sq<double2, S>);
     });
     with_square_side<float2>(sd, [&](auto side) {
@@ -1219,6 +1225,7 @@ int set_smem_limits() {
       for (const void* fn : {(const void*)k_zinv_sq<float2, S>, (const void*)k_zfwd_sq<float2, S>,
                              (const void*)k_xmid_sq<float2, S>, (const void*)k_xmid_dual_sq<float2, S>})
         limit(fn);
+      if constexpr (ZinvStaged<float2, S>::EVER) limit((const void*)k_zinv_staged<float2, S>);
       if constexpr (S % 2 == 0) limit((const void*)k_xmid_h2<float2, S>);
     });
   }

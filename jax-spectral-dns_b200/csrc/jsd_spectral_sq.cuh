@@ -2,7 +2,8 @@
 // (jsd_fftsq.cuh), used when the plan's FFT lengths are S * S. Same three
 // passes and the same intermediate layouts as the shared-memory kernels in
 // jsd_spectral.cuh, with one line per group of S lanes:
-//   k_zinv_sq : group per (y, kx): Hermitian part, 9 (18) inverse z transforms;
+//   k_zinv_sq : group per (y, kx): Hermitian part, 9 (18) inverse z transforms
+//               (k_zinv_staged: large boxes, input rows through shared memory);
 //   k_xmid_sq : block per (y, run of z columns), group per z column: packed
 //               pairs of fields through inverse x transforms, the products in
 //               registers (every lane owns the same x positions in every line),
@@ -132,6 +133,127 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __res
 template <typename C, int S>
 size_t zinv_sq_smem() {
   return sizeof(C) * (size_t)kSqWarps * SqLane<S>::G * sq_xbuf<S>();
+}
+
+// ---------------------------------------------------------------------------
+// inverse z pass, input rows staged (same output as k_zinv_sq, bit for bit): a
+// group's two rows (kx and -kx) of the next field come by cp.async into shared
+// memory while the transforms of the current one run, so a field's loads wait
+// for nothing; twiddles come from a shared table.
+// Bound: HBM, 4.5 TB/s at 129 x 129 modes x 129 planes in FP64 (what is left:
+// eight warps per SM alternate between transforms and line stores). Measured
+// there 98 us, 119 with k_zinv_sq's loads into registers; FP32 69 from 93; FP64
+// 161 x 161 x 145 169 from 257 (there the register loads spill).
+// The rows' way through shared memory costs 2 us where the fields lie in the
+// L2, so k_zinv_sq keeps boxes of fewer than kStagedMin entries per field (all
+// runs; six fields in and nine line sets out then share the L2): steps of 65 x
+// 65 x 89 modes 405 against 407 us, 29 x 19 x 85 150 against 158; above the line
+// 65 x 65 x 129 578 against 560, 97 x 97 x 97 1104 against 1061, four runs of 41 x
+// 97 x 41 623 against 600. FP64 S <= 7 stays with k_zinv_sq (twelve runs of 33 x 97
+// x 33 1166 against 1176), S = 16 is always staged (33 x 33 x 161 298 against 283).
+// ---------------------------------------------------------------------------
+constexpr size_t kStagedMin = 1u << 19;
+
+template <typename C, int S>
+struct ZinvStaged {
+  static constexpr bool F32 = sizeof(C) == sizeof(float2);
+  using Lane = SqLane<S, F32>;
+  static constexpr int GROUPS = kSqWarps * Lane::G, XB = sq_xbuf<S>(), TAB = (S - 1) * sq_tw_stride(S);
+  // whether the kernel is built for the side, and whether it then takes every box
+  static constexpr bool EVER = F32 ? S >= 7 : S >= 8, ALWAYS = !F32 && S == 16;
+  // registers: x, i kz x and the DFT's temporaries (238 at S = 14 in FP64: with
+  // three blocks it spills, 136 against 98 us)
+  static constexpr int BLOCKS = F32 ? 4 : S <= 10 ? 3 : 2;
+  // elements between the groups' row pairs: with consecutive-lane groups the
+  // lanes of a warp read one run of slots
+  static __host__ __device__ int row_stride(int mz) { return 2 * mz + ((S - 2 * mz) % 8 + 8) % 8; }
+  static size_t smem(const Geo& g) {
+    return sizeof(double2) * (size_t)GROUPS * row_stride(g.mz) + sizeof(C) * ((size_t)GROUPS * XB + TAB);
+  }
+};
+
+template <typename C, int S>
+__global__ void __launch_bounds__(kSqWarps * 32, ZinvStaged<C, S>::BLOCKS) k_zinv_staged(
+    Geo g, const C* __restrict__ twtab, ZinvSrc src, C* __restrict__ inter) {
+  using Z = ZinvStaged<C, S>;
+  using Rl = typename real_of<C>::type;
+  constexpr int N = S * S, TS = sq_tw_stride(S);
+  extern __shared__ __align__(16) unsigned char sq_raw[];
+  const typename Z::Lane ln;
+  const int group = ln.warp * Z::Lane::G + ln.gi, mz = g.mz;
+  double2* ra = reinterpret_cast<double2*>(sq_raw) + group * Z::row_stride(mz);
+  C* xb = reinterpret_cast<C*>(reinterpret_cast<double2*>(sq_raw) + Z::GROUPS * Z::row_stride(mz));
+  C* tab = xb + Z::GROUPS * Z::XB;
+  xb += group * Z::XB;
+  for (int e = threadIdx.x; e < Z::TAB; e += kSqWarps * 32) {
+    const int j = e / TS + 1, t = e % TS;
+    if (t < S) tab[e] = twtab[t * j];
+  }
+  const int K1 = g.kx_max + 1, K = g.kz_max;
+  const int pair = blockIdx.x * Z::GROUPS + group;
+  const bool act = ln.live && pair < g.ny * K1;
+  const int y = act ? pair / K1 : 0;
+  const int kx = act ? pair - y * K1 : 0;
+  const double2* rb = kx ? ra + mz : ra;  // the row of -kx
+  const size_t oa = sidx(g, y, kx, 0), ob = sidx(g, y, kx ? g.mx - kx : 0, 0);
+  // the group's rows of field i, by its own lanes
+  auto stage = [&](int i) {
+    if (act && i < 6 * src.nsets) {
+      const double2* f = zinv_field(src, i);
+#pragma unroll
+      for (int m = 0; m < S; ++m) {
+        const int p = ln.t + S * m;
+        if (p < mz) {
+          cp_async16(ra + p, f + oa + p, 16);
+          if (kx) cp_async16(ra + mz + p, f + ob + p, 16);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  pdl();
+  stage(0);
+  __syncthreads();  // the twiddle table
+#pragma unroll 1
+  for (int i = 0; i < 6 * src.nsets; ++i) {
+    const int set = i / 6, fi = i - 6 * set;
+    cp_async_wait<0>();
+    __syncwarp();
+    int t = ln.t;
+    asm volatile("" : "+r"(t));  // positions and wavenumbers formed here, not kept over the loop
+    C x[S], xz[S];
+    // K < N / 2: positions below N / 2 hold kz >= 0 modes, those above kz < 0
+#pragma unroll
+    for (int m = 0; m < S; ++m) {
+      const int p = t + S * m;
+      const bool below = S * m + S - 1 < N / 2, above = S * m >= N / 2;
+      const bool lo = !above && p <= K, hi = !below && p >= N - K;
+      const int kz = below ? p : above ? p - N : lo ? p : p - N;
+      C v = cmake<C>(0, 0);
+      if (act && (lo || hi)) {
+        const double2 a = ra[mode_pos(kz, mz)], b = rb[mode_pos(-kz, mz)];
+        v = to_c<C>(make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y)));
+      }
+      x[m] = v;
+      xz[m] = cmul_ik(v, (Rl)(kz * g.az));
+    }
+    __syncwarp();  // every lane has read the rows
+    stage(i + 1);
+    sq_fft_tab<S, true>(x, tab, xb, ln.t, ln.live);
+    C* o = inter + (((size_t)(set * kZinvLines + fi) * g.ny + y) * K1 + kx) * N + ln.t;
+    if (act) {
+#pragma unroll
+      for (int m = 0; m < S; ++m) o[S * m] = x[m];
+    }
+    if (fi < 3) {
+      sq_fft_tab<S, true>(xz, tab, xb, ln.t, ln.live);
+      C* oz = inter + (((size_t)(set * kZinvLines + 6 + fi) * g.ny + y) * K1 + kx) * N + ln.t;
+      if (act) {
+#pragma unroll
+        for (int m = 0; m < S; ++m) oz[S * m] = xz[m];
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
