@@ -389,14 +389,17 @@ def run_ours(args):
                 achieved = k["work"] / (k["ms"] / 1e3) / 1e12
                 mixed_sites = head == "mixed" and any(plans[head].eig_kernel(i)[0] == 1 for i in (1, 2))
                 label = ("k_dgemm + k_oz8_gemm (eigenbasis products: FP64 DMMA at one site, FP64-accurate "
-                         "int8 Ozaki at the other)" if mixed_sites else "k_dgemm (FP64 DMMA y-contractions)")
+                         "int8 Ozaki at the other)" if mixed_sites
+                         else "k_dgemm (FP64 DMMA y-contractions)" if head == "mixed"
+                         else "k_parity (FP64 DMMA y-contractions on even and odd parts: half the whole "
+                              "operators' operations, which `achieved` counts)")
                 roofline = {"kernel": label, "bound": "tensor",
                             "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                             "frac": achieved / fp64_peak,
                             "peak_source": "cuBLAS FP64 GEMM 8192^3 measured in this run (FP64 has no "
                                            "entry in MEASURED_PEAKS.json)",
                             "cublas_same_shape_tflops": same_shape,
-                            "traffic": _ncu_traffic("k_dgemm", head), "share_of_kernel_time": k["ms"] / total_k}
+                            "traffic": _ncu_traffic(label.split()[0], head), "share_of_kernel_time": k["ms"] / total_k}
             elif dom == "sgemm":
                 # split-TF32 products (y-derivatives, eigenbasis-in of the
                 # nonlinear terms): three TF32 tensor products per FP32-level
