@@ -756,6 +756,18 @@ __global__ void k_assemble_hv(Geo g, const double2* __restrict__ dq, const doubl
   }
 }
 
+// Parts of the field list of k_zinv_sq (grid rows): a box with few lines leaves
+// most SMs idle while each line's 9 (18) transforms run one after another, so the
+// fields are dealt to as many blocks as stay within about a wave and a half.
+// z pass at 33 x 33 modes x 65 planes (69 blocks) 14.6 -> 8.7 us with six parts,
+// 5 x 121 x 17 20.9 -> 10.7, 65 x 65 x 65 (179 blocks) 19.1 -> 16.8 with three;
+// beyond: 65 x 65 x 97 (267 blocks) 20.9 -> 21.9, 33 x 33 x 388 (412) 21.0 -> 21.3.
+int zinv_split(const jsd_plan* p, int blocks, int nsets) {
+  for (int parts : {6 * nsets, 6, 3})
+    if (4LL * blocks * parts <= 17LL * p->num_sms) return parts;
+  return 1;
+}
+
 template <typename C>
 int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2* conv, cudaStream_t s);
 
@@ -920,7 +932,7 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
             return;
           }
         if constexpr (!Z::ALWAYS)
-          run(k_zinv_sq<C, S>, blocks, kSqWarps * 32, zinv_sq_smem<C, S>(), s, g, tab, src, inter);
+          run(k_zinv_sq<C, S>, dim3(blocks, zinv_split(p, blocks, nsets)), kSqWarps * 32, zinv_sq_smem<C, S>(), s, g, tab, src, inter);
       });
       JSD_LAUNCHED("k_zinv_sq");
     } else {
@@ -940,8 +952,7 @@ int transforms(jsd_plan* p, const double2* state, const double2* uhist, double2*
       const C* tab = p->mixed ? (const C*)p->tsqz32 : (const C*)p->tsqz;
       with_square_side<C>(p->sqz, [&](auto side) {
         constexpr int S = decltype(side)::value;
-        const int per_block = kSqWarps * SqLane<S>::G;
-        run(k_zfwd_sq<C, S>, (ny * K1 + per_block - 1) / per_block, kSqWarps * 32, zfwd_sq_smem<C, S>(), s, g, tab,
+        run(k_zfwd_sq<C, S>, (ny * K1 + SqLane<S>::G - 1) / SqLane<S>::G, kZfwdThreads, zfwd_sq_smem<C, S>(), s, g, tab,
             out3, p->q, p->H1, p->hg, conv);
       });
       JSD_LAUNCHED("k_zfwd_sq");

@@ -63,7 +63,6 @@ __device__ __forceinline__ const double2* zinv_field(const ZinvSrc& src, int i) 
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __restrict__ twtab, ZinvSrc src,
                                                            C* __restrict__ inter) {
-  pdl();
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, XB = sq_xbuf<S>();
   // The two forms keep their best measured shapes: FP32 lines on half-warp
@@ -83,6 +82,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __res
   const int kx = act ? pair - y * K1 : 0;
   C tw[S - 1];
   sq_twiddles<S>(tw, twtab, ln.t);
+  pdl();
   // the group's two rows (kx and -kx) of field `i` into L2: the loads of a
   // field then wait for L2, not DRAM (one field ahead; rows are 16-byte
   // aligned and mz * 16 bytes long)
@@ -93,38 +93,37 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __res
       if (kx) l2_prefetch(f + sidx(g, y, g.mx - kx, 0), (unsigned)(g.mz * sizeof(double2)));
     }
   };
-  prefetch(1);
+  const int step = gridDim.y;
+  prefetch(blockIdx.y + step);
 #pragma unroll 1
-  for (int set = 0; set < src.nsets; ++set) {
-#pragma unroll 1
-    for (int fi = 0; fi < 6; ++fi) {
-      const double2* f = zinv_field(src, set * 6 + fi);
-      prefetch(set * 6 + fi + 2);
-      C x[S], xz[S];
-      // K < N / 2: positions below N / 2 hold kz >= 0 modes, those above kz < 0
+  for (int i = blockIdx.y; i < 6 * src.nsets; i += step) {
+    const int set = i / 6, fi = i - 6 * set;
+    const double2* f = zinv_field(src, i);
+    prefetch(i + 2 * step);
+    C x[S], xz[S];
+    // K < N / 2: positions below N / 2 hold kz >= 0 modes, those above kz < 0
 #pragma unroll
-      for (int m = 0; m < S; ++m) {
-        const int p = ln.t + S * m;
-        const bool below = F32 && S * m + S - 1 < N / 2, above = F32 && S * m >= N / 2;
-        const bool lo = !above && p <= K, hi = !below && p >= N - K;
-        const int kz = below ? p : above ? p - N : lo ? p : p - N;
-        const C v = (act && (lo || hi)) ? to_c<C>(sym_at(g, f, y, kx, kz)) : cmake<C>(0, 0);
-        x[m] = v;
-        xz[m] = cmul_ik(v, (Rl)(kz * g.az));
-      }
-      sq_fft<S, true>(x, tw, xb, ln.t, ln.live);
-      C* o = inter + (((size_t)(set * kZinvLines + fi) * g.ny + y) * K1 + kx) * N + ln.t;
+    for (int m = 0; m < S; ++m) {
+      const int p = ln.t + S * m;
+      const bool below = F32 && S * m + S - 1 < N / 2, above = F32 && S * m >= N / 2;
+      const bool lo = !above && p <= K, hi = !below && p >= N - K;
+      const int kz = below ? p : above ? p - N : lo ? p : p - N;
+      const C v = (act && (lo || hi)) ? to_c<C>(sym_at(g, f, y, kx, kz)) : cmake<C>(0, 0);
+      x[m] = v;
+      xz[m] = cmul_ik(v, (Rl)(kz * g.az));
+    }
+    sq_fft<S, true>(x, tw, xb, ln.t, ln.live);
+    C* o = inter + (((size_t)(set * kZinvLines + fi) * g.ny + y) * K1 + kx) * N + ln.t;
+    if (act) {
+#pragma unroll
+      for (int m = 0; m < S; ++m) o[S * m] = x[m];
+    }
+    if (fi < 3) {
+      sq_fft<S, true>(xz, tw, xb, ln.t, ln.live);
+      C* oz = inter + (((size_t)(set * kZinvLines + 6 + fi) * g.ny + y) * K1 + kx) * N + ln.t;
       if (act) {
 #pragma unroll
-        for (int m = 0; m < S; ++m) o[S * m] = x[m];
-      }
-      if (fi < 3) {
-        sq_fft<S, true>(xz, tw, xb, ln.t, ln.live);
-        C* oz = inter + (((size_t)(set * kZinvLines + 6 + fi) * g.ny + y) * K1 + kx) * N + ln.t;
-        if (act) {
-#pragma unroll
-          for (int m = 0; m < S; ++m) oz[S * m] = xz[m];
-        }
+        for (int m = 0; m < S; ++m) oz[S * m] = xz[m];
       }
     }
   }
@@ -259,40 +258,14 @@ __global__ void __launch_bounds__(kSqWarps * 32, ZinvStaged<C, S>::BLOCKS) k_zin
 // ---------------------------------------------------------------------------
 // forward z pass (same output as k_zfwd)
 // ---------------------------------------------------------------------------
+// Truncation and spectral combinations of a group's three transformed lines
+// lb[f * XB + position], by threads j, j + stride, ... of those that share it
 template <typename C, int S>
-__global__ void __launch_bounds__(kSqWarps * 32) k_zfwd_sq(Geo g, const C* __restrict__ twtab,
-                                                           const C* __restrict__ out3, double2* __restrict__ q,
-                                                           double2* __restrict__ H1, double2* __restrict__ hg,
-                                                           double2* __restrict__ conv00) {
-  pdl();
+__device__ __forceinline__ void zfwd_outputs(const Geo& g, const C* lb, int y, int kx, int j, int stride,
+                                             double2* __restrict__ q, double2* __restrict__ H1,
+                                             double2* __restrict__ hg, double2* __restrict__ conv00) {
   constexpr int N = S * S, XB = sq_xbuf<S>();
-  extern __shared__ __align__(16) unsigned char sq_raw[];
-  const SqLane<S> ln;
-  // three line buffers per group; the transforms exchange through line 0's
-  C* lb = reinterpret_cast<C*>(sq_raw) + (ln.warp * SqLane<S>::G + ln.gi) * 3 * XB;
-  const int K1 = g.kx_max + 1, K = g.kx_max;
-  const int pair = (blockIdx.x * kSqWarps + ln.warp) * SqLane<S>::G + ln.gi;
-  const bool act = ln.live && pair < g.ny * K1;
-  const int y = act ? pair / K1 : 0;
-  const int kx = act ? pair - y * K1 : 0;
-  C tw[S - 1];
-  sq_twiddles<S>(tw, twtab, ln.t);
-  // h1 and h2 first (parked in lines 1 and 2), h0 last (lands in line 0)
-#pragma unroll 1
-  for (int k = 0; k < 3; ++k) {
-    const int f = (k + 1) % 3;
-    const C* src = out3 + (((size_t)f * g.ny + y) * K1 + kx) * N + ln.t;
-    C x[S];
-#pragma unroll
-    for (int m = 0; m < S; ++m) x[m] = act ? src[S * m] : cmake<C>(0, 0);
-    sq_fft<S, false>(x, tw, lb, ln.t, ln.live);
-    if (ln.live) {
-#pragma unroll
-      for (int m = 0; m < S; ++m) lb[f * XB + ln.t + S * m] = x[m];
-    }
-  }
-  __syncwarp();
-  if (!act) return;
+  const int K = g.kx_max;
   const double cf = g.c_fwd;
   auto getF = [&](int f, int kz) -> double2 {
     const C v = lb[f * XB + (kz >= 0 ? kz : N + kz)];
@@ -304,7 +277,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zfwd_sq(Geo g, const C* __res
   rows[0] = kx;
   if (kx >= 1 && kx < K) rows[nrows++] = g.mx - kx;
   if (kx == K) rows[nrows++] = K + 1;
-  for (int i = ln.t; i < nrows * g.mz; i += S) {
+  for (int i = j; i < nrows * g.mz; i += stride) {
     const int rr = i >= g.mz ? 1 : 0;
     const int iz = i - rr * g.mz;
     const int ix = rows[rr];
@@ -321,9 +294,47 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_zfwd_sq(Geo g, const C* __res
   }
 }
 
+// Three warps per G line groups, each transforming one of a group's three lines;
+// then all of a group's lanes form the outputs. Bound: HBM in large boxes (181.9
+// MB in 41 us at 129 x 129 modes x 129 planes), one transform and the exchange in
+// small ones. One warp that transforms the three lines in turn and forms the
+// outputs takes 45 and, at 33 x 33 x 65, 10.7 us against 8.7; steps: 49 x 97 x 49
+// 336 -> 296 us, 161 x 145 x 161 3786 -> 3742, 129 x 129 x 129 2117 -> 2105.
+constexpr int kZfwdThreads = 96;
+
+template <typename C, int S>
+__global__ void __launch_bounds__(kZfwdThreads) k_zfwd_sq(Geo g, const C* __restrict__ twtab,
+                                                          const C* __restrict__ out3, double2* __restrict__ q,
+                                                          double2* __restrict__ H1, double2* __restrict__ hg,
+                                                          double2* __restrict__ conv00) {
+  constexpr int N = S * S, XB = sq_xbuf<S>();
+  extern __shared__ __align__(16) unsigned char sq_raw[];
+  const SqLane<S> ln;
+  C* lb = reinterpret_cast<C*>(sq_raw) + ln.gi * 3 * XB;
+  const int K1 = g.kx_max + 1, f = ln.warp;
+  const int pair = blockIdx.x * SqLane<S>::G + ln.gi;
+  const bool act = ln.live && pair < g.ny * K1;
+  const int y = act ? pair / K1 : 0;
+  const int kx = act ? pair - y * K1 : 0;
+  C tw[S - 1];
+  sq_twiddles<S>(tw, twtab, ln.t);
+  pdl();
+  const C* src = out3 + (((size_t)f * g.ny + y) * K1 + kx) * N + ln.t;
+  C x[S];
+#pragma unroll
+  for (int m = 0; m < S; ++m) x[m] = act ? src[S * m] : cmake<C>(0, 0);
+  sq_fft<S, false>(x, tw, lb + f * XB, ln.t, ln.live);
+  if (ln.live) {
+#pragma unroll
+    for (int m = 0; m < S; ++m) lb[f * XB + ln.t + S * m] = x[m];
+  }
+  __syncthreads();
+  if (act) zfwd_outputs<C, S>(g, lb, y, kx, ln.t + S * f, 3 * S, q, H1, hg, conv00);
+}
+
 template <typename C, int S>
 size_t zfwd_sq_smem() {
-  return sizeof(C) * (size_t)kSqWarps * SqLane<S>::G * 3 * sq_xbuf<S>();
+  return sizeof(C) * (size_t)SqLane<S>::G * 3 * sq_xbuf<S>();
 }
 
 // ---------------------------------------------------------------------------

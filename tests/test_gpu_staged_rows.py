@@ -51,3 +51,19 @@ def test_dual_sets(cuda):
     want, gain, _, _ = O.dual_gradient(shape, LX, LZ, RE, DT, n, u0, False)
     assert rel(grad.cpu().numpy(), want) < 1e-10
     assert abs(g / gain - 1) < 1e-10
+
+
+@pytest.mark.parametrize("runs", [48, 49, 98, 99])
+def test_parts_of_the_field_list(cuda, runs):
+    """Block counts on both sides of the lines between six, three and one part
+    of the field list (24 lines per block: 102, 105, 209 and 211 blocks)."""
+    shape = (4, 17, 16)
+    modes, phys = mode_counts(shape)
+    base = 1 - cheb_points(shape[1]) ** 2
+    u = seeded_velocity_hat(shape, (LX, LZ), (2, 8), 1e-3, seed=runs)
+    plan = StepPlan(modes, phys, LX, LZ, 1, [RE] * runs, DT, base_u=base)
+    st = pack_runs([u] * runs)
+    plan.step(st, torch.zeros(1, dtype=torch.float64, device="cuda"), 0, 1)
+    want, _, _ = O.run(O.make_stepper("perturbation", shape, LX, LZ, RE, DT, linearise=False), u, 1)
+    for got in unpack_runs(st):
+        assert rel(got.cpu().numpy(), want) < 1e-10
