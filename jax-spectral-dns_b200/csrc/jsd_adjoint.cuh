@@ -31,9 +31,9 @@ namespace jsd {
 // omega_y (non-(0,0) modes, interior rows) and of the mean-flow solution
 // (x00: u00 then w00 per Chebyshev point; zero at the walls, which the forward
 // step overwrites).
-__global__ void k_reconstruct_adj(Geo g, const double2* __restrict__ lu, const double2* __restrict__ lw,
-                                  double2* __restrict__ dv_bar, double2* __restrict__ om_bar,
-                                  double2* __restrict__ x00_bar) {
+__global__ void k_reconstruct_adj(Geo g, const double2* lu, const double2* lw,
+                                  double2* dv_bar, double2* om_bar,
+                                  double2* x00_bar) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -112,11 +112,11 @@ __device__ __forceinline__ void mean_flow_adj_block(const Geo& g, const MeanFlow
 // and ny-1 of wall_out, a spectral field whose interior rows the caller fills
 // later); and in hv_old / hg_old the cotangents of the previous stage's terms.
 __global__ void __launch_bounds__(kEigCols * kEigParts, 4) k_eigen_update_adj(
-    Geo g, EigTables t, StageCoef sc, MeanFlowAdj mf, int last, const double* __restrict__ vn_bar_a,
-    const double* __restrict__ vn_bar_b, const double* __restrict__ omn_bar, double* __restrict__ hv_old,
-    double* __restrict__ hg_old, double* __restrict__ X1_bar, double* __restrict__ T0_bar,
-    double* __restrict__ T1_bar, double* __restrict__ vt_bar, double* __restrict__ omt_bar,
-    double* __restrict__ wall_out) {
+    Geo g, EigTables t, StageCoef sc, MeanFlowAdj mf, int last, const double* vn_bar_a,
+    const double* vn_bar_b, const double* omn_bar, double* hv_old,
+    double* hg_old, double* X1_bar, double* T0_bar,
+    double* T1_bar, double* vt_bar, double* omt_bar,
+    double* wall_out) {
   pdl();
   if ((int)blockIdx.x < mf.blocks) {
     mean_flow_adj_block(g, mf, blockIdx.x);
@@ -264,12 +264,12 @@ __device__ __forceinline__ int sources_of(const Geo& g, int pm, int kmax, int m,
   return 1;
 }
 
-__global__ void k_linear_terms_adj(Geo g, const double* __restrict__ ubase, const double* __restrict__ dubase,
-                                   const double2* __restrict__ qb, const double2* __restrict__ H1b,
-                                   const double2* __restrict__ hgb, const double2* __restrict__ convb,
-                                   const double2* __restrict__ omb, const double2* __restrict__ vextra,
-                                   const double2* __restrict__ x00, double2* __restrict__ lu,
-                                   double2* __restrict__ lv, double2* __restrict__ lw, double2* __restrict__ dvb) {
+__global__ void k_linear_terms_adj(Geo g, const double* ubase, const double* dubase,
+                                   const double2* qb, const double2* H1b,
+                                   const double2* hgb, const double2* convb,
+                                   const double2* omb, const double2* vextra,
+                                   const double2* x00, double2* lu,
+                                   double2* lv, double2* lw, double2* dvb) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -328,7 +328,7 @@ __global__ void k_linear_terms_adj(Geo g, const double* __restrict__ ubase, cons
   }
 }
 
-__global__ void k_add_field(size_t n, const double2* __restrict__ a, double2* __restrict__ out) {
+__global__ void k_add_field(size_t n, const double2* a, double2* out) {
   pdl();
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
     out[t] = cadd(out[t], a[t]);
@@ -338,8 +338,8 @@ __global__ void k_add_field(size_t n, const double2* __restrict__ a, double2* __
 // sum_y w_y sum |Sym f|^2 over the three components, s = c_inv^2 / 4) with
 // respect to the real and imaginary parts of every coefficient: 2 s w_y Sym f
 // (Sym, the Hermitian part, is an orthogonal projection).
-__global__ void k_energy_grad(Geo g, const double2* __restrict__ f, const double* __restrict__ w, double scale2,
-                              double2* __restrict__ out) {
+__global__ void k_energy_grad(Geo g, const double2* f, const double* w, double scale2,
+                              double2* out) {
   pdl();
   const size_t fs = (size_t)g.ny * g.nk;
   const size_t total = 3 * fs;

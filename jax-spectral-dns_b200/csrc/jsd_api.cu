@@ -743,8 +743,8 @@ Geo planes_of(const Geo& g) {
 }
 
 // h_v = -D q - k^2 H1 (only for the nonlinear-term hook)
-__global__ void k_assemble_hv(Geo g, const double2* __restrict__ dq, const double2* __restrict__ h1,
-                              double2* __restrict__ hv) {
+__global__ void k_assemble_hv(Geo g, const double2* dq, const double2* h1,
+                              double2* hv) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {

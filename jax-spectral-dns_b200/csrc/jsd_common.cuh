@@ -82,7 +82,12 @@ __host__ __device__ __forceinline__ size_t sidx(const Geo& g, int y, int ix, int
 // reads, so a kernel that is done implies that all before it are. In this order
 // at most the next kernel is resident early, and none starts while a kernel two
 // before it still fills caches. Only tables fixed at plan creation may be read
-// before the wait.
+// before the wait. For the same reason the kernels' parameters that point to
+// data carry no __restrict__: it would say of the whole kernel, the time before
+// the wait included, that nothing else writes that memory, and let the compiler
+// load it early. It bought nothing: registers are alike but in two kernels, two
+// steps of 129 x 129 x 129 take 4421 us without it and 4435 with it, a linear step
+// of 9 x 65 x 5 66.2 and 66.7.
 __device__ __forceinline__ void pdl_trigger() {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -280,7 +280,7 @@ __device__ __forceinline__ double oz_i2d(uint32_t x) {
 #endif
 
 __global__ void __launch_bounds__(kOzThreads, 1) k_oz8_gemm(const __grid_constant__ OzBatch b,
-                                                             int* __restrict__ err, int spin) {
+                                                             int* err, int spin) {
   pdl();
 #if defined(__CUDA_ARCH__)
   extern __shared__ unsigned char osm_raw[];

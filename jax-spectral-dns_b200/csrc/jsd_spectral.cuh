@@ -42,7 +42,7 @@ struct ZinvSrc {
 };
 
 template <typename C>
-__global__ void k_zinv(Geo g, FftDesc fz, const C* __restrict__ tw, ZinvSrc src, C* __restrict__ inter) {
+__global__ void k_zinv(Geo g, FftDesc fz, const C* __restrict__ tw, ZinvSrc src, C* inter) {
   pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char zsm_raw[];
@@ -175,9 +175,9 @@ __device__ __forceinline__ void forward_and_store(const Geo& g, const FftDesc& f
 
 template <typename C, int ZB>
 __global__ void __launch_bounds__(kXmidThreads) k_xmid(Geo g, FftDesc fx, const C* __restrict__ tw,
-                                                       const C* __restrict__ inter, C* __restrict__ out3,
-                                                       const double* __restrict__ ubase,
-                                                       const double* __restrict__ dubase, double lam_d) {
+                                                       const C* inter, C* out3,
+                                                       const double* ubase,
+                                                       const double* dubase, double lam_d) {
   pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char xsm_raw[];
@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(kXmidThreads) k_xmid(Geo g, FftDesc fx, const 
 // ---------------------------------------------------------------------------
 template <typename C, int ZB>
 __global__ void __launch_bounds__(kXmidThreads) k_xmid_dual(Geo g, FftDesc fx, const C* __restrict__ tw,
-                                                            const C* __restrict__ inter, C* __restrict__ out3,
-                                                            const double* __restrict__ ubase,
-                                                            const double* __restrict__ dubase) {
+                                                            const C* inter, C* out3,
+                                                            const double* ubase,
+                                                            const double* dubase) {
   pdl();
   using Rl = typename real_of<C>::type;
   extern __shared__ __align__(16) unsigned char xsm_raw[];
@@ -372,9 +372,9 @@ __device__ __forceinline__ void write_terms(const Geo& g, int y, int ix, int iz,
 // forcing -conv00 + s00 takes s00 through conv00 -= s00. The source is fixed
 // over the three stages of a step, so the old terms of the next stage carry it
 // as the reference's do.
-__global__ void k_add_source(Geo g, const double2* __restrict__ hv, const double2* __restrict__ hgs,
-                             const double2* __restrict__ s00, double2* __restrict__ H1, double2* __restrict__ hg,
-                             double2* __restrict__ conv00) {
+__global__ void k_add_source(Geo g, const double2* hv, const double2* hgs,
+                             const double2* s00, double2* H1, double2* hg,
+                             double2* conv00) {
   pdl();
   const size_t n = (size_t)g.ny * g.nk, n00 = 2 * (size_t)g.ny;
   const size_t total = n > n00 ? n : n00;
@@ -402,8 +402,8 @@ __global__ void k_add_source(Geo g, const double2* __restrict__ hv, const double
 // as at every other wavenumber (navier_stokes.py:1697-1703). One thread per
 // eigen row; single-run plans (the source is one field).
 template <typename TI>
-__global__ void k_add_source00(Geo g, const double* __restrict__ vinv, int lda, const double2* __restrict__ hv,
-                               TI* __restrict__ X1) {
+__global__ void k_add_source00(Geo g, const double* __restrict__ vinv, int lda, const double2* hv,
+                               TI* X1) {
   pdl();
   const int n = g.ny - 2;
   const size_t N = 2 * (size_t)g.nk * g.nb;
@@ -422,9 +422,9 @@ __global__ void k_add_source00(Geo g, const double* __restrict__ vinv, int lda, 
 
 // forward z pass: block (kx in [0, K], y).
 template <typename C>
-__global__ void k_zfwd(Geo g, FftDesc fz, const C* __restrict__ tw, const C* __restrict__ out3,
-                       double2* __restrict__ q, double2* __restrict__ H1, double2* __restrict__ hg,
-                       double2* __restrict__ conv00) {
+__global__ void k_zfwd(Geo g, FftDesc fz, const C* __restrict__ tw, const C* out3,
+                       double2* q, double2* H1, double2* hg,
+                       double2* conv00) {
   pdl();
   extern __shared__ __align__(16) unsigned char fsm_raw[];
   C* fsm = reinterpret_cast<C*>(fsm_raw);
@@ -502,11 +502,11 @@ __device__ __forceinline__ void linear_pre(const Geo& g, const double2* __restri
 }
 
 template <int KIND>
-__global__ void k_linear_terms(Geo g, const double2* __restrict__ u, const double2* __restrict__ v,
-                               const double2* __restrict__ w, const double2* __restrict__ dv,
-                               const double* __restrict__ ubase, const double* __restrict__ dubase,
-                               double2* __restrict__ q, double2* __restrict__ H1, double2* __restrict__ hg,
-                               double2* __restrict__ conv00) {
+__global__ void k_linear_terms(Geo g, const double2* u, const double2* v,
+                               const double2* w, const double2* dv,
+                               const double* ubase, const double* dubase,
+                               double2* q, double2* H1, double2* hg,
+                               double2* conv00) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -538,8 +538,8 @@ __global__ void k_linear_terms(Geo g, const double2* __restrict__ u, const doubl
 //                 streamwise component of the dual field.
 // g.ny = planes (batch runs included); dubase indexed by Chebyshev row.
 template <int KIND>
-__global__ void k_coupling_off(Geo g, const double2* __restrict__ f, const double* __restrict__ dubase,
-                               double2* __restrict__ H1, double2* __restrict__ hg) {
+__global__ void k_coupling_off(Geo g, const double2* f, const double* dubase,
+                               double2* H1, double2* hg) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -561,8 +561,8 @@ __global__ void k_coupling_off(Geo g, const double2* __restrict__ f, const doubl
 }
 
 // omega_y = i kz u - i kx w (the y component of curl u, domain.py:920-933)
-__global__ void k_omega(Geo g, const double2* __restrict__ u, const double2* __restrict__ w,
-                        double2* __restrict__ om) {
+__global__ void k_omega(Geo g, const double2* u, const double2* w,
+                        double2* om) {
   pdl();
   const size_t total = (size_t)g.ny * g.nk;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -691,10 +691,10 @@ inline size_t eigen_update_smem(int ny, int parts) {
 // products (the mixed form). The first mf.blocks * g.nb blocks are the mean flow's.
 template <typename TI, int PARTS>
 __global__ void __launch_bounds__(kEigCols * PARTS, PARTS > kEigParts ? 2 : 4) k_eigen_update(
-    Geo g, EigTables t, StageCoef sc, MeanFlow mf, const TI* __restrict__ X1, const TI* __restrict__ H1t,
-    const TI* __restrict__ hgt, const double* __restrict__ vt, const double* __restrict__ omt,
-    const double* __restrict__ vfield, TI* __restrict__ hv_old, TI* __restrict__ hg_old,
-    double* __restrict__ vnt, double* __restrict__ omnt, int rpp) {
+    Geo g, EigTables t, StageCoef sc, MeanFlow mf, const TI* X1, const TI* H1t,
+    const TI* hgt, const double* vt, const double* omt,
+    const double* vfield, TI* hv_old, TI* hg_old,
+    double* vnt, double* omnt, int rpp) {
   pdl();
   constexpr bool KEEP = PARTS > kEigParts;
   __shared__ double red[PARTS][6][kEigCols];
@@ -821,9 +821,9 @@ __global__ void __launch_bounds__(kEigCols * PARTS, PARTS > kEigParts ? 2 : 4) k
 // u, w of the new state from continuity, the (0,0) mean flow and the wall
 // rows; raises kErrNonFinite in `err` when any value it reads (dv/dy, omega_y
 // and the mean flow, from which all of u, v, w follow) is not finite.
-__global__ void k_reconstruct(Geo g, const double2* __restrict__ dvn, const double2* __restrict__ omn,
-                              const double2* __restrict__ uw00, double2* __restrict__ u, double2* __restrict__ v,
-                              double2* __restrict__ w, int* __restrict__ err) {
+__global__ void k_reconstruct(Geo g, const double2* dvn, const double2* omn,
+                              const double2* uw00, double2* u, double2* v,
+                              double2* w, int* err) {
   pdl();
   const size_t total = (size_t)g.ny * g.nb * g.nk;
   bool bad = false;
@@ -902,8 +902,8 @@ __global__ void k_weighted_total(int ny, const double* __restrict__ weights, con
 // slice]. Same terms as k_plane_sums, summed in a fixed order.
 constexpr int kSumSlices = 8;
 
-__global__ void __launch_bounds__(256) k_plane_sums_sliced(Geo g, const double2* __restrict__ f, int ncomp, int mode,
-                                                          double* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_plane_sums_sliced(Geo g, const double2* f, int ncomp, int mode,
+                                                          double* out) {
   pdl();
   const int y = blockIdx.x, slice = blockIdx.y;
   const int chunk = (g.nk + kSumSlices - 1) / kSumSlices;
@@ -951,7 +951,7 @@ __device__ __forceinline__ double weighted_slices(int ny, int stride, int offset
 
 // out = scale * sum over planes (single run), one warp
 __global__ void k_weighted_total_sliced(int ny, const double* __restrict__ weights,
-                                        const double* __restrict__ partial, double scale, double* __restrict__ out) {
+                                        const double* partial, double scale, double* out) {
   pdl();
   const double a = weighted_slices(ny, 1, 0, weights, partial);
   if (threadIdx.x == 0) out[0] = scale * a;
@@ -959,8 +959,8 @@ __global__ void k_weighted_total_sliced(int ny, const double* __restrict__ weigh
 
 // per-run totals of a batch: one warp per run
 __global__ void k_weighted_total_runs_sliced(int ny, int nb, const double* __restrict__ weights,
-                                             const double* __restrict__ partial, double scale,
-                                             double* __restrict__ out) {
+                                             const double* partial, double scale,
+                                             double* out) {
   pdl();
   const int run = blockIdx.x;
   const double a = weighted_slices(ny, nb, run, weights, partial);
@@ -975,8 +975,8 @@ __global__ void k_weighted_total_runs_sliced(int ny, int nb, const double* __res
 // the same order, block 0 updates dPdx. u in place: a thread owns the entries at
 // (+-kx, +-kz), which are all that the round trip of any of them reads.
 __global__ void __launch_bounds__(256) k_mass_flux(Geo g, const double* __restrict__ weights,
-                                                   const double* __restrict__ partial, double q0, double dt_e,
-                                                   double* __restrict__ dpdx, double2* __restrict__ u) {
+                                                   const double* partial, double q0, double dt_e,
+                                                   double* dpdx, double2* u) {
   pdl();
   __shared__ double off;
   if (threadIdx.x < 32) {

@@ -62,7 +62,7 @@ __device__ __forceinline__ const double2* zinv_field(const ZinvSrc& src, int i) 
 // ---------------------------------------------------------------------------
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32) k_zinv_sq(Geo g, const C* __restrict__ twtab, ZinvSrc src,
-                                                           C* __restrict__ inter) {
+                                                           C* inter) {
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, XB = sq_xbuf<S>();
   // The two forms keep their best measured shapes: FP32 lines on half-warp
@@ -173,7 +173,7 @@ struct ZinvStaged {
 
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32, ZinvStaged<C, S>::BLOCKS) k_zinv_staged(
-    Geo g, const C* __restrict__ twtab, ZinvSrc src, C* __restrict__ inter) {
+    Geo g, const C* __restrict__ twtab, ZinvSrc src, C* inter) {
   using Z = ZinvStaged<C, S>;
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, TS = sq_tw_stride(S);
@@ -304,9 +304,9 @@ constexpr int kZfwdThreads = 96;
 
 template <typename C, int S>
 __global__ void __launch_bounds__(kZfwdThreads) k_zfwd_sq(Geo g, const C* __restrict__ twtab,
-                                                          const C* __restrict__ out3, double2* __restrict__ q,
-                                                          double2* __restrict__ H1, double2* __restrict__ hg,
-                                                          double2* __restrict__ conv00) {
+                                                          const C* out3, double2* q,
+                                                          double2* H1, double2* hg,
+                                                          double2* conv00) {
   constexpr int N = S * S, XB = sq_xbuf<S>();
   extern __shared__ __align__(16) unsigned char sq_raw[];
   const SqLane<S> ln;
@@ -519,9 +519,9 @@ constexpr int xsq_min_blocks() {
 //   hel_i = -lam (u . grad) u_i + lam/2 (div u) u_i - U d_x u_i - delta_i0 (v U' - (div u) U / 2)
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32, xsq_min_blocks<C>()) k_xmid_sq(Geo g, const C* __restrict__ twtab,
-                                                           const C* __restrict__ inter, C* __restrict__ out3,
-                                                           const double* __restrict__ ubase,
-                                                           const double* __restrict__ dubase, double lam_d) {
+                                                           const C* inter, C* out3,
+                                                           const double* ubase,
+                                                           const double* dubase, double lam_d) {
   pdl();
   using Rl = typename real_of<C>::type;
   constexpr int G = SqLane<S>::G, ZC = XmidSq<C, S>::ZC, XB = sq_xbuf<S>();
@@ -614,9 +614,9 @@ __global__ void __launch_bounds__(kSqWarps * 32, xsq_min_blocks<C>()) k_xmid_sq(
 // Intermediate lines 0..8 hold v (v, dv/dy, dv/dz), 9..17 the same for u.
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_dual_sq(Geo g, const C* __restrict__ twtab,
-                                                                const C* __restrict__ inter, C* __restrict__ out3,
-                                                                const double* __restrict__ ubase,
-                                                                const double* __restrict__ dubase) {
+                                                                const C* inter, C* out3,
+                                                                const double* ubase,
+                                                                const double* dubase) {
   pdl();
   using Rl = typename real_of<C>::type;
   constexpr int G = SqLane<S>::G, ZC = XmidSq<C, S>::ZC, XB = sq_xbuf<S>();
@@ -752,9 +752,9 @@ __device__ __forceinline__ void xh2_fill(const Geo& g, const C* tile, int zl, in
 
 template <typename C, int S>
 __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __restrict__ twtab,
-                                                           const C* __restrict__ inter, C* __restrict__ out3,
-                                                           const double* __restrict__ ubase,
-                                                           const double* __restrict__ dubase, double lam_d) {
+                                                           const C* inter, C* out3,
+                                                           const double* ubase,
+                                                           const double* dubase, double lam_d) {
   pdl();
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, H = S / 2, G = SqLane2<S>::G, ZC = XmidH2<C, S>::ZC, XB = sq_xbuf<S>();
@@ -1010,10 +1010,10 @@ __device__ __forceinline__ double2 xpark_value(const double2* mode, double side,
 
 template <class P>
 __global__ void __launch_bounds__(kSqWarps * 32, P::BLOCKS) k_xmid_park(Geo g, const double2* __restrict__ twtab,
-                                                                        const double2* __restrict__ inter,
-                                                                        double2* __restrict__ out3,
-                                                                        const double* __restrict__ ubase,
-                                                                        const double* __restrict__ dubase) {
+                                                                        const double2* inter,
+                                                                        double2* out3,
+                                                                        const double* ubase,
+                                                                        const double* dubase) {
   pdl();
   using X = XmidPark<P>;
   constexpr int S = P::S, N = S * S, R = P::R, G = P::G, ZC = X::ZC, XB = P::XB;

@@ -217,7 +217,7 @@ __device__ __forceinline__ double tc_load_if(const double* p, bool c) {
 #endif
 
 __global__ void __launch_bounds__(kTcThreads, 1) k_tc05_split(const __grid_constant__ Tc05Batch b,
-                                                              int* __restrict__ err, int spin) {
+                                                              int* err, int spin) {
   pdl();
 #if defined(__CUDA_ARCH__)
   extern __shared__ __align__(1024) unsigned char tsm[];
