@@ -228,20 +228,32 @@ size_t jsd_workspace_bytes(const jsd_plan* plan);
  * the plan's three GEMM call sites (y-derivatives, eigenbasis transforms in,
  * back-transforms out) with the plan's own sizes and workspace, and keeps the
  * fastest per site, and likewise chooses among the x-pass kernel variants of
- * the nonlinear terms. Overwrites workspace only (no state); synchronises the
+ * the nonlinear terms. Sites whose products run on even and odd parts
+ * (jsd_even_odd_products) stay in that form, also where jsd_set_gemm_config had
+ * set a tile. Overwrites workspace only (no state); synchronises the
  * stream, so it must not be called during stream capture. */
 int jsd_autotune(jsd_plan* plan, void* stream);
 
-/* Tile configuration in use at GEMM call site `site` (0 y-derivatives,
- * 1 eigenbasis in, 2 eigenbasis out), or -1 for a bad argument; if times_ms is
+/* Tile configuration at GEMM call site `site` (0 y-derivatives, 1 eigenbasis
+ * in, 2 eigenbasis out) for products with whole operators, or -1 for a bad
+ * argument (whether the site runs such products: jsd_even_odd_products); if times_ms is
  * not null it receives the autotuner's per-configuration times (7 floats, 0
  * for configurations not timed). */
 int jsd_gemm_config(const jsd_plan* plan, int site, float* times_ms);
 
-/* Use tile configuration `config` (0..6) at GEMM call site `site`. Every
+/* Use tile configuration `config` (0..6) at GEMM call site `site`, which then
+ * runs products with whole operators until jsd_autotune is called. Every
  * configuration sums over K in the same order, so results do not depend on
- * the choice. No counterpart in the reference. */
+ * which is set; products on even and odd parts sum in another order and differ
+ * by round-off. No counterpart in the reference. */
 int jsd_set_gemm_config(jsd_plan* plan, int site, int config);
+
+/* 1 when GEMM call site `site` runs its products on the even and odd parts of
+ * the profiles (two products of half the size; the form of FP64 plans of 10 to
+ * 194 points whose operator tables have definite parity, where neither a tile nor the
+ * int8 kernel is set for the site), 0 when it runs whole operators, -1 for a
+ * bad argument. No counterpart in the reference. */
+int jsd_even_odd_products(const jsd_plan* plan, int site);
 
 /* x-pass kernel of the nonlinear terms in use: 0 register FFT with S lanes per
  * x line, 1 register FFT with 2 S lanes per line, 2 shared-memory FFT; if

@@ -241,6 +241,7 @@ struct jsd_plan {
   double* re_run = nullptr;     // Reynolds number per run of a batch (device)
   double* lr_ns = nullptr;      // Linv_ns R_ns per run and stage (row-parallel mean-flow update)
   int gemm_cfg[3] = {2, 2, 2};  // DMMA tile configuration per call site (GemmSite)
+  bool gemm_set[3] = {};        // the caller set the site's tile: it runs whole operators in it, not k_parity
   int xmid_variant = 2;         // x-pass kernel (launch_xmid), set at creation, autotuned on request
   float xmid_ms[3] = {};        // autotuner timings of the x-pass variants (0: not timed)
   float tune_ms[3][kDgemmConfigs] = {};  // autotuner timings per site and configuration (0: not timed)
@@ -572,10 +573,10 @@ bool with_parity_shape(int w, int tm, F&& f) {
   return false;
 }
 
-// The batch on even and odd parts; false when an entry's operator has no such
-// form or the entries differ in what they fold.
-bool parity_batch(const jsd_plan* p, const GemmBatch& b, ParityBatch& o, bool& fold) {
-  if (!p->par_w || b.count < 1 || b.ldb != b.N || b.ldc != b.N) return false;
+// The batch on even and odd parts; false when the caller set a tile for the
+// site, an entry's operator has no such form or the entries differ in what they fold.
+bool parity_batch(const jsd_plan* p, const GemmBatch& b, GemmSite site, ParityBatch& o, bool& fold) {
+  if (!p->par_w || p->gemm_set[site] || b.count < 1 || b.ldb != b.N || b.ldc != b.N) return false;
   memset(&o, 0, sizeof(o));
   o.N = b.N;
   o.count = b.count;
@@ -625,7 +626,7 @@ int launch_gemm(const jsd_plan* p, const GemmBatch& b, int max_m, GemmSite site,
   ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, gemm_flops(b), s);
   ParityBatch o;
   bool fold = false;
-  if (parity_batch(p, b, o, fold)) return launch_parity(p, o, fold, s);
+  if (parity_batch(p, b, site, o, fold)) return launch_parity(p, o, fold, s);
   return launch_gemm_cfg(p, b, max_m, p->gemm_cfg[site], s);
 }
 
@@ -1164,7 +1165,7 @@ int stage_adj(jsd_plan* p, double2* lam, int st, bool last, cudaStream_t s) {
     add_entry(b, p->D_T, (const double*)(p->Dfld + fs), (double*)lv, ny, ny);
     ParityBatch o;
     bool fold = false;
-    if (parity_batch(p, b, o, fold)) {
+    if (parity_batch(p, b, kSiteDfield, o, fold)) {
       o.accumulate = 1;
       return launch_parity(p, o, fold, s);
     }
@@ -1376,6 +1377,7 @@ int jsd_autotune(jsd_plan* plan, void* stream) {
   JSD_CUDA(cudaEventCreate(&e0));
   JSD_CUDA(cudaEventCreate(&e1));
   int rc = 0;
+  for (bool& set : plan->gemm_set) set = false;  // the choice is the plan's again
   for (int site = 0; site < kGemmSites && rc == 0; ++site) {
     if (site == kSiteDfield && plan->mixed) continue;  // the mixed form's y-derivatives run k_sgemm3
     GemmBatch b = gemm_batch(plan);
@@ -1592,7 +1594,13 @@ int jsd_set_gemm_config(jsd_plan* plan, int site, int config) {
   if (!plan || site < 0 || site >= kGemmSites || config < 0 || config >= kDgemmConfigs)
     return fail(JSD_ERR_ARG, "bad GEMM site or configuration");
   plan->gemm_cfg[site] = config;
+  plan->gemm_set[site] = true;
   return 0;
+}
+
+int jsd_even_odd_products(const jsd_plan* plan, int site) {
+  if (!plan || site < 0 || site >= kGemmSites) return -1;
+  return plan->par_w && !plan->gemm_set[site] && !(plan->oz_ready && plan->eig_kernel[site] == 1) ? 1 : 0;
 }
 
 int jsd_gemm_config(const jsd_plan* plan, int site, float* times_ms) {

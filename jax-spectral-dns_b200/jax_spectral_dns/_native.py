@@ -49,7 +49,7 @@ EXPORTED = (
     "jsd_workspace_bytes", "jsd_launches_per_step", "jsd_last_error", "jsd_abi_version",
     "jsd_profile_enable", "jsd_profile_read", "jsd_energy_noalloc", "jsd_step_trajectory",
     "jsd_launches_first_step_extra", "jsd_autotune", "jsd_gemm_config",
-    "jsd_set_gemm_config", "jsd_xmid_variant", "jsd_set_xmid_variant",
+    "jsd_set_gemm_config", "jsd_even_odd_products", "jsd_xmid_variant", "jsd_set_xmid_variant",
     "jsd_energy_runs", "jsd_set_batch_active", "jsd_batch_active",
     "jsd_split_kernel", "jsd_set_split_kernel", "jsd_split_eig_in", "jsd_set_split_eig_in", "jsd_device_error",
     "jsd_set_coupling_term", "jsd_set_base_flow", "jsd_eig_kernel", "jsd_set_eig_kernel",
@@ -116,6 +116,7 @@ def load(path: str = LIB_PATH):
     lib.jsd_autotune.argtypes = [vp, vp]
     lib.jsd_gemm_config.argtypes = [vp, ctypes.c_int, ctypes.POINTER(ctypes.c_float)]
     lib.jsd_set_gemm_config.argtypes = [vp, ctypes.c_int, ctypes.c_int]
+    lib.jsd_even_odd_products.argtypes = [vp, ctypes.c_int]
     lib.jsd_xmid_variant.argtypes = [vp, ctypes.POINTER(ctypes.c_float)]
     lib.jsd_energy_runs.argtypes = [vp, vp, vp, vp]
     lib.jsd_split_kernel.argtypes = [vp, ctypes.POINTER(ctypes.c_float)]

@@ -130,15 +130,21 @@ class StepPlan:
 
     def autotune(self) -> dict:
         """Time every FP64 tensor-core tile configuration at each GEMM call site
-        on this plan's sizes and keep the fastest (jsd_autotune)."""
+        on this plan's sizes and keep the fastest; sites whose products run on
+        even and odd parts stay so (jsd_autotune)."""
         with torch.cuda.device(self.device):
             _native.check(self.lib.jsd_autotune(self.handle, _stream_ptr()), "jsd_autotune")
             torch.cuda.synchronize(self.device)
         return self.gemm_configs()
 
     def set_gemm_config(self, site: str, config: int) -> None:
+        """Run whole operators in tile `config` at a GEMM call site (jsd_set_gemm_config)."""
         _native.check(self.lib.jsd_set_gemm_config(self.handle, _native.GEMM_SITES[site], int(config)),
                       "jsd_set_gemm_config")
+
+    def even_odd_products(self, site: str) -> bool:
+        """Whether a GEMM call site runs its products on even and odd parts."""
+        return self.lib.jsd_even_odd_products(self.handle, _native.GEMM_SITES[site]) == 1
 
     def xmid_variant(self):
         """(x-pass variant in use, [autotune ms of variants 0, 1, 2])."""
