@@ -255,10 +255,14 @@ int jsd_set_gemm_config(jsd_plan* plan, int site, int config);
  * bad argument. No counterpart in the reference. */
 int jsd_even_odd_products(const jsd_plan* plan, int site);
 
-/* x-pass kernel of the nonlinear terms in use: 0 register FFT with S lanes per
- * x line, 1 register FFT with 2 S lanes per line, 2 shared-memory FFT; if
- * times_ms is not null it receives the autotuner's times of the three (0 for
- * variants not timed or not available). No counterpart in the reference. */
+/* x-pass kernel of the nonlinear terms in use, for the FFT length S * S. Mixed
+ * form: 0 register FFT with S lanes per x line, 1 register FFT with 2 S lanes
+ * per line (even S, not the dual), 2 shared-memory FFT. FP64 form: 0 (S <= 7)
+ * and 1 (even S, or S > 7) both name its one register kernel (S lanes per line
+ * up to S = 10, 2 S beyond; the dual has 0 only, S <= 7), 2 shared-memory FFT.
+ * If times_ms is not null it receives the autotuner's times of the three (0 for
+ * variants not timed: not available, or 0 where 1 is the same kernel). No
+ * counterpart in the reference. */
 int jsd_xmid_variant(const jsd_plan* plan, float* times_ms);
 
 /* Force x-pass variant 0, 1 or 2 (JSD_ERR_ARG when it does not apply to the

@@ -840,6 +840,11 @@ bool xmid_available(const jsd_plan* p, int v) {
   return false;
 }
 
+// 0 and 1 name one kernel (FP64, not the dual, sides 4 and 6): only 1 is timed.
+bool xmid_alias(const jsd_plan* p, int v) {
+  return v == 0 && !p->mixed && p->desc.kind != JSD_KIND_DUAL && xmid_available(p, 1);
+}
+
 int default_xmid_variant(const jsd_plan* p) {
   if (p->mixed && xmid_available(p, 0)) return 0;
   if (xmid_available(p, 1)) return 1;
@@ -1479,7 +1484,8 @@ int jsd_autotune(jsd_plan* plan, void* stream) {
   if (rc == 0 && !linear) {
     float best = 3.0e38f;
     for (int v = 0; v < 3 && rc == 0; ++v) {
-      if (!xmid_available(plan, v)) continue;
+      plan->xmid_ms[v] = 0.f;
+      if (!xmid_available(plan, v) || xmid_alias(plan, v)) continue;
       auto run = [&]() {
         return plan->mixed ? launch_xmid<float2>(plan, v, (float2*)plan->inter, (float2*)plan->out3, s)
                            : launch_xmid<double2>(plan, v, (double2*)plan->inter, (double2*)plan->out3, s);
