@@ -27,9 +27,11 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <vector>
 
+#include "../../include/jsd.h"
 #include "jsd_common.cuh"
 #include "jsd_gemm.cuh"
 
@@ -101,6 +103,78 @@ inline std::vector<double> parity_pack(const std::vector<double>& h, int M, int 
       else out[parity_slot(row_tiles, r, k)] = v;
     }
   return out;
+}
+
+// The eigenbasis tables of a plan with every eigenvector exactly even or odd
+// and the even modes first (the order of the eigen rows is the plan's own),
+// and D exactly odd under y -> -y. An eigenvector as a solver returns it has
+// the other parity mixed in at the level its eigenvalue's neighbour allows
+// (7e-11 at Ny = 129), D is odd to its own round-off (5e-15 of its largest
+// entry; its first rows are kept and mirrored, so rows still sum to zero). The
+// boundary vectors belong to the same tables: kept from the unsymmetrised ones,
+// w0 differs from D[0, int] V by 8e-11 of itself at Ny = 129.
+struct SymTables {
+  bool ok = false;
+  int n_even = 0;
+  std::vector<double> D, V, Vinv, lam, sgn, c0, cN, w0, wN;
+};
+
+inline SymTables symmetric_tables(const jsd_desc* d) {
+  SymTables t;
+  const int ny = d->ny, n = ny - 2;
+  auto D = [&](int r, int c) { return d->D[(size_t)r * ny + c]; };
+  auto V = [&](int r, int c) { return d->V[(size_t)r * n + c]; };
+  auto W = [&](int r, int c) { return d->Vinv[(size_t)r * n + c]; };
+  double dmax = 0, vmax = 0, wmax = 0;
+  for (int i = 0; i < ny * ny; ++i) dmax = std::max(dmax, std::fabs(d->D[i]));
+  for (int i = 0; i < n * n; ++i) {
+    vmax = std::max(vmax, std::fabs(d->V[i]));
+    wmax = std::max(wmax, std::fabs(d->Vinv[i]));
+  }
+  std::vector<int> order;
+  for (int want : {1, -1})
+    for (int j = 0; j < n; ++j)
+      if (d->sgn[j] == want) order.push_back(j);
+  if ((int)order.size() != n) return t;
+  for (int j = 0; j < n; ++j) t.n_even += d->sgn[j] == 1;
+  if (t.n_even != (n + 1) / 2) return t;
+  // (comparisons written so that a NaN fails them)
+  for (int r = 0; r < ny; ++r)
+    for (int c = 0; c < ny; ++c)
+      if (!(std::fabs(D(r, c) + D(ny - 1 - r, ny - 1 - c)) <= 1e-10 * dmax)) return t;
+  for (int r = 0; r < n; ++r)
+    for (int c = 0; c < n; ++c)
+      if (!(std::fabs(V(r, c) - d->sgn[c] * V(n - 1 - r, c)) <= 1e-8 * vmax) ||
+          !(std::fabs(W(r, c) - d->sgn[r] * W(r, n - 1 - c)) <= 1e-8 * wmax))
+        return t;
+  t.ok = true;
+  t.D.resize((size_t)ny * ny);
+  for (int r = 0; r < ny; ++r)
+    for (int c = 0; c < ny; ++c)
+      t.D[(size_t)r * ny + c] = 2 * r < ny - 1   ? D(r, c)
+                                : 2 * r > ny - 1 ? -D(ny - 1 - r, ny - 1 - c)
+                                                 : 0.5 * (D(r, c) - D(r, ny - 1 - c));
+  t.V.resize((size_t)n * n);
+  t.Vinv.resize((size_t)n * n);
+  for (int j = 0; j < n; ++j) {
+    const int o = order[j];
+    for (int r = 0; r < n; ++r) {
+      t.V[(size_t)r * n + j] = 0.5 * (V(r, o) + d->sgn[o] * V(n - 1 - r, o));
+      t.Vinv[(size_t)j * n + r] = 0.5 * (W(o, r) + d->sgn[o] * W(o, n - 1 - r));
+    }
+    const double sg = d->sgn[o];
+    t.lam.push_back(d->lam[o]);
+    t.sgn.push_back(sg);
+    // the boundary columns of D^2 mirror each other, so the new rows of V^-1 give
+    // the definite part of (c0, cN); w0 and wN are formed again from the new D, V
+    t.c0.push_back(0.5 * (d->c0[o] + sg * d->cN[o]));
+    t.cN.push_back(sg * t.c0[j]);
+    long double w = 0;
+    for (int r = 0; r < n; ++r) w += (long double)t.D[r + 1] * t.V[(size_t)r * n + j];
+    t.w0.push_back((double)w);
+    t.wN.push_back(-sg * t.w0[j]);
+  }
+  return t;
 }
 
 // Halves of a whole operator A (mout x kin, row-major). fold / unfold: its
