@@ -82,11 +82,6 @@ def _peaks():
         return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}, "fallback"
 
 
-# kernel class -> summary file stem under profiles/ (<stem>_channel_128x129x128.md)
-KERNEL_NAMES = {"gemm": "k_dgemm", "sgemm": "k_tc05_split", "zinv": "k_zinv_sq", "xmid": "k_xmid", "zfwd": "k_zfwd_sq",
-                "eigen": "k_eigen_update"}
-
-
 def _ncu_traffic(kernel: str, form: str):
     """DRAM bytes (read + write) per launch of `kernel` from the committed ncu
     summary of the benchmark workload, or None when there is none."""
@@ -104,6 +99,95 @@ def _ncu_traffic(kernel: str, form: str):
         return float(vals[form]) * 1e6
     launches = [float(v) for k, v in vals.items() if k.startswith("launch")]
     return sum(launches) / len(launches) * 1e6 if launches else None
+
+
+def kernel_of(cls: str, form: str, choices: dict):
+    """Name of the kernel that a class of the benchmark box's plan runs, or
+    None where the class runs two. choices: eig_kernel (sites in, out),
+    even_odd (the three call sites), split_kernel, xmid_variant."""
+    if cls == "gemm":
+        int8 = [k == 1 for k in choices["eig_kernel"]]
+        if form == "mixed":
+            return "k_oz8_gemm" if all(int8) else None if any(int8) else "k_dgemm"
+        if any(int8):
+            return None
+        return "k_parity" if all(choices["even_odd"]) else None if any(choices["even_odd"]) else "k_dgemm"
+    if cls == "xmid":
+        return (("k_xmid_sq", "k_xmid_h2", "k_xmid") if form == "mixed" else
+                ("k_xmid_park", "k_xmid_park", "k_xmid"))[choices["xmid_variant"]]
+    if cls == "sgemm":
+        return "k_tc05_split" if choices["split_kernel"] == 1 else "k_sgemm3"
+    # zinv: more than half a million entries per field
+    return {"zinv": "k_zinv_staged", "zfwd": "k_zfwd_sq", "eigen": "k_eigen_update"}[cls]
+
+
+# What the kernel's label says beside its name, and what limits a pass whose bytes do not
+LABELS = {"k_oz8_gemm": "FP64-accurate eigenbasis products, Ozaki int8 on tcgen05",
+          "k_dgemm": "FP64 DMMA y-contractions",
+          "k_parity": "FP64 DMMA y-contractions on even and odd parts",
+          "k_tc05_split": "split-TF32 products on tcgen05", "k_sgemm3": "split-TF32 products, mma.sync"}
+LIMITERS = {"k_xmid_sq": "instruction issue (ncu: 63% issue active, 12 warps per SM, 92 M warp instructions per launch; "
+                         "profiles/k_xmid_sq_channel_128x129x128.md)",
+            "k_xmid_park": "shared-memory wavefronts (ncu: 67% of the pipe, FP64 pipe 34%; "
+                           "profiles/k_xmid_park_channel_128x129x128.md)"}
+
+
+def roofline_line(dom, kernels, form, choices, modes, peaks, peak_src, fp64=None):
+    """Roofline entry of the dominant kernel class: its rate (of the operations
+    that its kernel executes, or of its algorithmic bytes) over the peak of what
+    bounds it. fp64: measured (cuBLAS FP64 GEMM peak, cuBLAS rate at the product's
+    own shape, whole operators), TFLOP/s; needed for the class "gemm"."""
+    k = kernels[dom]
+    kernel = kernel_of(dom, form, choices)
+    name = (kernel + (f" ({LABELS[kernel]})" if kernel in LABELS else "")) if kernel else {
+        "mixed": "k_dgemm + k_oz8_gemm (eigenbasis products: FP64 DMMA at one site, FP64-accurate int8 Ozaki at the other)",
+        "fp64": "k_parity / k_dgemm / k_oz8_gemm (y-contractions: another kernel at each call site)"}[form]
+    out = {"kernel": name}
+    if dom == "gemm":
+        peak, same_shape = fp64
+        achieved = k["work"] / (k["ms"] / 1e3) / 1e12
+        out.update(bound="tensor", achieved=achieved, peak=peak, unit="TFLOP/s", frac=achieved / peak,
+                   peak_source="cuBLAS FP64 GEMM 8192^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json)")
+        ny = modes[1]
+        if kernel == "k_oz8_gemm":
+            # the mixed form's eigenbasis products on the int8 tensor cores:
+            # FP64-equivalent throughput against the FP64 GEMM peak they
+            # replace, and the int8 pipe's own use (36 slice products of 128 x
+            # 128 tensor tiles per FP64-equivalent (Ny-2) x Ny product)
+            int8_tops = achieved * 36 * 128 * 128 / ((ny - 2) * ny)
+            int8_peak = 2 * peaks["bf16_tflops"]
+            out.update(unit="TFLOP/s (FP64-equivalent)",
+                       int8_pipe={"achieved_tops": int8_tops, "peak_tops": int8_peak, "frac": int8_tops / int8_peak,
+                                  "peak_source": "2 x bf16_tflops of MEASURED_PEAKS.json (dense int8 issues at twice "
+                                                 "the bf16 rate)"})
+        else:
+            out["cublas_same_shape_tflops"] = same_shape
+        if kernel == "k_parity":
+            # two products of half the size stand for one: the rate of whole
+            # operators that they replace (at the (Ny-2) x Ny shape), beside the executed one
+            m, n = ny - 2, ny
+            executed = ((m + 1) // 2) * (n // 2) + (m // 2) * ((n + 1) // 2)
+            out["whole_operator_equivalent_tflops"] = achieved * m * n / executed
+    elif dom == "sgemm":
+        # split-TF32 products (y-derivatives, eigenbasis-in of the nonlinear
+        # terms): three TF32 tensor products per FP32-level product, against
+        # the dense TF32 rate (half the bf16 rate)
+        achieved, peak = 3 * k["work"] / (k["ms"] / 1e3) / 1e12, peaks["bf16_tflops"] / 2
+        out.update(bound="tensor", achieved=achieved, peak=peak, unit="TFLOP/s (TF32)", frac=achieved / peak,
+                   peak_source=peak_src + " (MEASURED_PEAKS.json bf16_tflops / 2)")
+    else:
+        achieved, peak = k["work"] / (k["ms"] / 1e3) / 1e9, peaks["hbm_gbs"]
+        out.update(bound="hbm", achieved=achieved, peak=peak, unit="GB/s", frac=achieved / peak,
+                   peak_source=peak_src + " (MEASURED_PEAKS.json hbm_gbs)",
+                   algorithmic_bytes_per_launch=k["work"] / k["launches"])
+        if kernel in LIMITERS:
+            out["limiter"] = LIMITERS[kernel]  # the pass's bytes are small next to its FFT arithmetic
+    out["traffic"] = _ncu_traffic(kernel, form) if kernel else None
+    out["share_of_kernel_time"] = k["ms"] / sum(v["ms"] for v in kernels.values())
+    if out["traffic"] is not None:
+        out["traffic_source"] = ("dram__bytes per launch (read + write), "
+                                 f"profiles/{kernel}_channel_128x129x128.md")
+    return out
 
 
 class ClockSampler:
@@ -255,6 +339,7 @@ def run_ours(args):
     dev = torch.device("cuda", local)
     if world > 1:
         dist.init_process_group("nccl", timeout=__import__("datetime").timedelta(seconds=300))
+    from jax_spectral_dns import _native
     from jax_spectral_dns._plan import GraphedSteps, StepPlan, to_device_layout, to_reference_layout
     from jax_spectral_dns.seeds import mode_counts
 
@@ -359,75 +444,14 @@ def run_ours(args):
         total_k = sum(v["ms"] for v in kernels.values())
         roofline = None
         if dom is not None:
-            k = kernels[dom]
-            ozaki = head == "mixed" and all(plans[head].eig_kernel(i)[0] == 1 for i in (1, 2))
-            if dom == "gemm" and ozaki:
-                # the mixed form's only GEMM-class launches are the eigenbasis
-                # products, here on the int8 tensor cores: FP64-equivalent
-                # throughput against the FP64 GEMM peak they replace, and the
-                # int8 pipe's own use (36 slice products of 128 x 128 tensor
-                # tiles per FP64-equivalent (Ny-2) x Ny product)
-                fp64_peak = measure_fp64_peak(dev)
-                achieved = k["work"] / (k["ms"] / 1e3) / 1e12
-                ny = modes[1]
-                int8_tops = achieved * 36 * 128 * 128 / ((ny - 2) * ny)
-                int8_peak = 2 * peaks["bf16_tflops"]
-                roofline = {"kernel": "k_oz8_gemm (FP64-accurate eigenbasis products, Ozaki int8 on tcgen05)",
-                            "bound": "tensor", "achieved": achieved, "peak": fp64_peak,
-                            "unit": "TFLOP/s (FP64-equivalent)", "frac": achieved / fp64_peak,
-                            "peak_source": "cuBLAS FP64 GEMM 8192^3 measured in this run (FP64 has no "
-                                           "entry in MEASURED_PEAKS.json)",
-                            "int8_pipe": {"achieved_tops": int8_tops, "peak_tops": int8_peak,
-                                          "frac": int8_tops / int8_peak,
-                                          "peak_source": "2 x bf16_tflops of MEASURED_PEAKS.json (dense int8 "
-                                                         "issues at twice the bf16 rate)"},
-                            "traffic": _ncu_traffic("k_oz8_gemm", head), "share_of_kernel_time": k["ms"] / total_k}
-            elif dom == "gemm":
-                fp64_peak = measure_fp64_peak(dev)
-                ny = modes[1]
-                same_shape = measure_fp64_same_shape(dev, ny - 2, ny, 3 * 2 * modes[0] * modes[2])
-                achieved = k["work"] / (k["ms"] / 1e3) / 1e12
-                mixed_sites = head == "mixed" and any(plans[head].eig_kernel(i)[0] == 1 for i in (1, 2))
-                label = ("k_dgemm + k_oz8_gemm (eigenbasis products: FP64 DMMA at one site, FP64-accurate "
-                         "int8 Ozaki at the other)" if mixed_sites
-                         else "k_dgemm (FP64 DMMA y-contractions)" if head == "mixed"
-                         else "k_parity (FP64 DMMA y-contractions on even and odd parts: half the whole "
-                              "operators' operations, which `achieved` counts)")
-                roofline = {"kernel": label, "bound": "tensor",
-                            "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                            "frac": achieved / fp64_peak,
-                            "peak_source": "cuBLAS FP64 GEMM 8192^3 measured in this run (FP64 has no "
-                                           "entry in MEASURED_PEAKS.json)",
-                            "cublas_same_shape_tflops": same_shape,
-                            "traffic": _ncu_traffic(label.split()[0], head), "share_of_kernel_time": k["ms"] / total_k}
-            elif dom == "sgemm":
-                # split-TF32 products (y-derivatives, eigenbasis-in of the
-                # nonlinear terms): three TF32 tensor products per FP32-level
-                # product, against the dense TF32 rate (half the bf16 rate)
-                achieved = 3 * k["work"] / (k["ms"] / 1e3) / 1e12
-                tf32_peak = peaks["bf16_tflops"] / 2
-                roofline = {"kernel": "k_tc05_split (split-TF32 products on tcgen05)", "bound": "tensor",
-                            "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s (TF32)",
-                            "frac": achieved / tf32_peak,
-                            "peak_source": peak_src + " (MEASURED_PEAKS.json bf16_tflops / 2)",
-                            "traffic": _ncu_traffic("k_tc05_split", head),
-                            "share_of_kernel_time": k["ms"] / total_k}
-            else:
-                achieved = k["work"] / (k["ms"] / 1e3) / 1e9
-                roofline = {"kernel": KERNEL_NAMES[dom], "bound": "hbm", "achieved": achieved,
-                            "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
-                            "peak_source": peak_src + " (MEASURED_PEAKS.json hbm_gbs)",
-                            "traffic": _ncu_traffic(KERNEL_NAMES[dom], head),
-                            "algorithmic_bytes_per_launch": k["work"] / k["launches"],
-                            "share_of_kernel_time": k["ms"] / total_k}
-                if dom == "xmid":
-                    # its bytes are small next to its FFT arithmetic: the HBM
-                    # fraction is low because instruction issue limits it
-                    roofline["limiter"] = ("instruction issue (ncu: 62% issue active, 12 warps per SM, 92 M warp "
-                                           "instructions per launch; profiles/k_xmid_channel_128x129x128.md)")
-            if roofline["traffic"] is not None:
-                roofline["traffic_source"] = ("dram__bytes_read.sum + dram__bytes_write.sum per launch, "
-                                              f"profiles/{roofline['kernel'].split()[0]}_channel_128x129x128.md")
+            choices = {"eig_kernel": [plans[head].eig_kernel(i)[0] for i in (1, 2)],
+                       "even_odd": [plans[head].even_odd_products(site) for site in _native.GEMM_SITES],
+                       "split_kernel": plans[head].split_kernel()[0],
+                       "xmid_variant": plans[head].xmid_variant()[0]}
+            fp64 = (measure_fp64_peak(dev),
+                    measure_fp64_same_shape(dev, modes[1] - 2, modes[1], 3 * 2 * modes[0] * modes[2])
+                    ) if dom == "gemm" else None
+            roofline = roofline_line(dom, kernels, head, choices, modes, peaks, peak_src, fp64)
         per_kernel = {k: {"avg_us": round(1e3 * v["ms"] / v["launches"], 2), "launches": v["launches"],
                           "share": round(v["ms"] / total_k, 4)} for k, v in kernels.items()}
         for k, v in kernels.items():
@@ -437,6 +461,7 @@ def run_ours(args):
                 per_kernel[k]["gbs"] = round(v["work"] / (v["ms"] / 1e3) / 1e9, 1)
         # side legs and kernel choices on their own lines, before the headline
         details = {pr: {"gemm_configs": {site: cfg for site, (cfg, _) in plans[pr].gemm_configs().items()},
+                        "even_odd_products": {site: plans[pr].even_odd_products(site) for site in _native.GEMM_SITES},
                         "split_kernel": plans[pr].split_kernel(), "split_eig_in": plans[pr].split_eig_in(),
                         "xmid_variant": plans[pr].xmid_variant(),
                         "eig_kernels": {site: plans[pr].eig_kernel(i) for i, site in ((1, "eig_in"), (2, "eig_out"))}}

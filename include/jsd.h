@@ -326,7 +326,9 @@ int jsd_launches_first_step_extra(const jsd_plan* plan);
 /* Optional timing of kernel classes with CUDA events (no effect unless
  * enabled). jsd_profile_read returns and clears, for one class, the summed
  * device time (ms), the number of launches and the summed algorithmic work
- * (FLOPs for JSD_PROF_GEMM, bytes for the others). No reference counterpart. */
+ * (bytes, but FLOPs for JSD_PROF_GEMM and JSD_PROF_SGEMM: those of the products
+ * as they run, on even and odd parts half the whole operators'). No reference
+ * counterpart. */
 enum jsd_prof_class {
   JSD_PROF_GEMM = 0,    /* FP64 y-contractions (DMMA) */
   JSD_PROF_ZINV = 1,    /* inverse z transforms */

@@ -607,7 +607,16 @@ bool parity_batch(const jsd_plan* p, const GemmBatch& b, GemmSite site, ParityBa
   return true;
 }
 
+// operations of the two half-size products of every entry
+double parity_flops(const ParityBatch& o) {
+  double f = 0;
+  for (int i = 0; i < o.count; ++i)
+    for (int h = 0; h < 2; ++h) f += 2.0 * o.e[i].M[h] * (double)o.e[i].K[h] * o.N;
+  return f;
+}
+
 int launch_parity(const jsd_plan* p, ParityBatch& o, bool fold, cudaStream_t s) {
+  ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, parity_flops(o), s);
   o.rows = parity_rows(o, fold, parity_ksteps(p->par_w * p->par_tm));
   const long long tiles = (long long)((o.N + kParN - 1) / kParN) * o.count;
   with_parity_shape(p->par_w, p->par_tm, [&](auto W, auto TM) {
@@ -623,10 +632,10 @@ int launch_parity(const jsd_plan* p, ParityBatch& o, bool fold, cudaStream_t s) 
 }
 
 int launch_gemm(const jsd_plan* p, const GemmBatch& b, int max_m, GemmSite site, cudaStream_t s) {
-  ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, gemm_flops(b), s);
   ParityBatch o;
   bool fold = false;
   if (parity_batch(p, b, site, o, fold)) return launch_parity(p, o, fold, s);
+  ProfScope ps(const_cast<jsd_plan*>(p), JSD_PROF_GEMM, gemm_flops(b), s);
   return launch_gemm_cfg(p, b, max_m, p->gemm_cfg[site], s);
 }
 

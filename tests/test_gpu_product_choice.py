@@ -92,3 +92,34 @@ def test_adjoint_is_the_transpose_in_either_form(cuda, ny, tiles):
     plan.step_adjoint(sty, 1)
     dot = lambda a, b: torch.sum(a.real * b.real + a.imag * b.imag).item()  # noqa: E731
     assert abs(dot(sx, y) - dot(x, sty)) < 1e-12 * (sx.abs().norm() * y.abs().norm()).item()
+
+
+@pytest.mark.parametrize("ny", [10, 33, 34, 195])
+@pytest.mark.parametrize("tiles", [False, True])
+def test_profile_counts_the_operations_that_run(cuda, ny, tiles):
+    """FLOPs of the product class over one step: D on three (first stage) or two
+    fields, three products into the eigenbasis and one more in the first stage
+    (V^-1 omega_y) with V^-1 v, three out of it; on even and odd parts each whole
+    product M x K counts M / 2 x K / 2 twice (halves rounded up and down)."""
+    plan = _plan(ny)
+    if tiles:
+        for site in _native.GEMM_SITES:
+            plan.set_gemm_config(site, 0)
+    plan.profile(True)
+    _step(plan, ny, 1)
+    _, _, work = plan.profile_read("gemm")
+    plan.profile(False)
+    mx, _, mz = plan.modes
+    halves = 10 <= ny <= 194 and not tiles
+
+    def product(m, k, crossed):
+        if not halves:
+            return m * k
+        (me, mo), (ke, ko) = ((m + 1) // 2, m // 2), ((k + 1) // 2, k // 2)
+        return me * ko + mo * ke if crossed else me * ke + mo * ko
+
+    n = ny - 2
+    d, vd, vi, v, dv = (product(ny, ny, True), product(n, ny, True), product(n, n, False), product(ny, n, False),
+                        product(ny, n, True))
+    fields = (3 + 2 + 2) * d + 3 * (vd + 2 * vi + 2 * v + dv) + 2 * vi
+    assert work == 2.0 * fields * 2 * mx * mz
