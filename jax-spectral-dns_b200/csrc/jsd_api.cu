@@ -266,7 +266,7 @@ struct jsd_plan {
   int par_w = 0, par_tm = 0;  // kernel shape (0: no parity products)
   int n_even = 0;             // even modes: eigen rows 0 .. n_even - 1
   double *lam = nullptr, *sgn = nullptr, *c0 = nullptr, *cN = nullptr, *w0 = nullptr, *wN = nullptr;
-  double *yw = nullptr, *rhs_ns = nullptr, *lhs_inv_ns = nullptr, *ub = nullptr, *dub = nullptr;
+  double *yw = nullptr, *lhs_inv_ns = nullptr, *ub = nullptr, *dub = nullptr;
   // workspace
   double2 *Dfld = nullptr;     // 3 fields: D u, D v, D w
   void *inter = nullptr;       // 9 (18 for the dual) z-transformed lines per (y, kx >= 0)
@@ -1946,7 +1946,6 @@ int jsd_plan_create(const jsd_desc* d, jsd_plan** out) {
   JSD_TRY(upload(p, &p->w0, d->w0, ni));
   JSD_TRY(upload(p, &p->wN, d->wN, ni));
   JSD_TRY(upload(p, &p->yw, d->y_weights, ny));
-  JSD_TRY(upload(p, &p->rhs_ns, d->rhs_ns, (size_t)nb * 3 * n2 * n2));
   JSD_TRY(upload(p, &p->lhs_inv_ns, d->lhs_inv_ns, (size_t)nb * 3 * n2 * n2));
   if (nb > 1) JSD_TRY(upload(p, &p->re_run, d->re_tau_batch, (size_t)nb));
   {
