@@ -12,10 +12,11 @@
 // between an inverse and a forward transform stays in registers, and the only
 // synchronisation is a __syncwarp around the exchange.
 //
-// S-point DFTs in registers: radices 2, 3, 4, 5, 7, 8 directly (jsd_fft.cuh),
-// composite S with coprime factors by the prime-factor (Good-Thomas) mapping,
-// which needs no twiddles: n = (B n1 + A n2) mod S, k = (B (B^-1 mod A) k1 +
-// A (A^-1 mod B) k2) mod S for S = A B.
+// S-point DFTs in registers: radices 2, 3, 4, 5, 7, 8 directly (jsd_fft.cuh), 9
+// and 16 as squares of 3 and 4 with twiddles (dft_square), composite S with
+// coprime factors by the prime-factor (Good-Thomas) mapping, which needs no
+// twiddles: n = (B n1 + A n2) mod S, k = (B (B^-1 mod A) k1 + A (A^-1 mod B)
+// k2) mod S for S = A B.
 #pragma once
 
 #include "jsd_common.cuh"
@@ -33,10 +34,6 @@ __host__ __device__ constexpr int sq_inv_mod(int a, int m) {
 __host__ __device__ constexpr int sq_split(int s) {
   return s == 6 ? 2 : s == 10 ? 2 : s == 12 ? 4 : s == 14 ? 2 : s == 15 ? 3 : s == 20 ? 4 : s == 21 ? 3
        : s == 24 ? 8 : s == 28 ? 4 : s == 30 ? 2 : 0;
-}
-
-__host__ __device__ constexpr bool sq_supported(int s) {
-  return s == 2 || s == 3 || s == 4 || s == 5 || s == 7 || s == 8 || s == 9 || s == 16 || sq_split(s) != 0;
 }
 
 template <int R, bool INV, typename C>

@@ -4,12 +4,14 @@
 // jsd_spectral.cuh, with one line per group of S lanes:
 //   k_zinv_sq : group per (y, kx): Hermitian part, 9 (18) inverse z transforms
 //               (k_zinv_staged: large boxes, input rows through shared memory);
-//   k_xmid_sq : block per (y, run of z columns), group per z column: packed
-//               pairs of fields through inverse x transforms, the products in
+//   k_xmid_sq : mixed form: block per (y, run of z columns), group per z column:
+//               packed pairs of fields through inverse x transforms, the products in
 //               registers (every lane owns the same x positions in every line),
-//               2 forward x transforms;
-//   k_zfwd_sq : group per (y, kx): 3 forward z transforms, truncation and the
-//               spectral combinations of write_terms.
+//               2 forward x transforms (k_xmid_h2: the line on 2 S lanes);
+//   k_xmid_park : the same for the FP64 form, finished components in shared
+//               memory, columns across planes (k_xmid_dual_sq: the dual's);
+//   k_zfwd_sq : group per (y, kx) on three warps, one forward z transform each,
+//               then truncation and the spectral combinations of write_terms.
 // All sizes are compile-time, so index arithmetic is shifts and multiplies,
 // and the only synchronisation inside a transform is a __syncwarp.
 #pragma once
@@ -508,20 +510,17 @@ __device__ __forceinline__ void xsq_store(const Geo& g, const C* otile, C* __res
 }
 
 // Resident blocks per SM the FP32 x pass is compiled for (registers capped at
-// 168 per lane: a little spilling, 12 warps per SM instead of 8). The FP64 form
-// runs k_xmid_park.
-template <typename C>
-constexpr int xsq_min_blocks() {
-  return sizeof(C) == sizeof(float2) ? 3 : 1;
-}
+// 168 per lane: a little spilling, 12 warps per SM instead of 8).
+constexpr int kXsqBlocks = 3;
 
-// NS / perturbation products, as in k_xmid:
+// NS / perturbation products of the mixed form (the FP64 form runs k_xmid_park), as in k_xmid:
 //   hel_i = -lam (u . grad) u_i + lam/2 (div u) u_i - U d_x u_i - delta_i0 (v U' - (div u) U / 2)
 template <typename C, int S>
-__global__ void __launch_bounds__(kSqWarps * 32, xsq_min_blocks<C>()) k_xmid_sq(Geo g, const C* __restrict__ twtab,
+__global__ void __launch_bounds__(kSqWarps * 32, kXsqBlocks) k_xmid_sq(Geo g, const C* __restrict__ twtab,
                                                            const C* inter, C* out3,
                                                            const double* ubase,
                                                            const double* dubase, double lam_d) {
+  static_assert(sizeof(C) == sizeof(float2), "FP64 lines: k_xmid_park");
   pdl();
   using Rl = typename real_of<C>::type;
   constexpr int G = SqLane<S>::G, ZC = XmidSq<C, S>::ZC, XB = sq_xbuf<S>();
@@ -686,8 +685,10 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_dual_sq(Geo g, const C* 
 }
 
 // ---------------------------------------------------------------------------
-// x pass, half-split lanes (even S): a z column's lines on 2 S lanes, H = S / 2
-// points per lane (sq2_fft). Half the registers per lane of k_xmid_sq.
+// x pass of the mixed form, half-split lanes (even S): a z column's lines on 2 S
+// lanes, H = S / 2 points per lane (sq2_fft). Half the registers per lane of
+// k_xmid_sq; the autotuner's alternative to it (129 x 129 modes x 129 planes: 172 us
+// against 134).
 // ---------------------------------------------------------------------------
 template <int S>
 struct SqLane2 {
@@ -755,6 +756,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __res
                                                            const C* inter, C* out3,
                                                            const double* ubase,
                                                            const double* dubase, double lam_d) {
+  static_assert(sizeof(C) == sizeof(float2), "FP64 lines: k_xmid_park");
   pdl();
   using Rl = typename real_of<C>::type;
   constexpr int N = S * S, H = S / 2, G = SqLane2<S>::G, ZC = XmidH2<C, S>::ZC, XB = sq_xbuf<S>();
