@@ -77,7 +77,9 @@ typedef struct jsd_desc {
   const double* rhs_ns;    /* [3*(2ny)^2] (0,0) explicit matrices per RK stage (navier_stokes.py:1000-1022) */
   const double* lhs_inv_ns;/* [3*(2ny)^2] (0,0) implicit inverses per RK stage */
   int precision;           /* JSD_PRECISION_FP64, or JSD_PRECISION_MIXED: FP32 transforms and products,
-                              split-TF32 tensor-core y-derivatives; solves stay FP64 */
+                              split-TF32 tensor-core y-derivatives; solves stay FP64. Mixed is the
+                              faster form from about 0.6 million entries per field (65 x 97 x 105) to
+                              129 modes a side; FP64 is faster below, and again beyond 129 modes */
   /* Batch of independent runs on the same box (no counterpart in the
    * reference, which steps one field at a time). n_batch <= 1: one run.
    * n_batch > 1: every field holds the runs side by side, plane by plane,

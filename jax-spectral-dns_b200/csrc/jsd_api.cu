@@ -306,8 +306,10 @@ namespace {
 // of 474, 97 x 97 x 97 (0.9 M entries per field) 2305 instead of 2434. From
 // fields that no longer share the L2 on they lose (129 x 129 x 129, 2.1 M entries:
 // 4706 against 4593), and in a captured graph, whose nodes already follow each
-// other closely, they cost 1 us per node (270 nodes at 33 x 65 x 33: 1892 us
-// against 1630), so both keep plain order. The mixed form loses much earlier
+// other closely, they cost 1 us per node (ten steps of 27 launches at 33 x 65 x 33:
+// 1892 us against 1630), so both keep plain order. Below the line the size alone
+// does not decide it: 33 x 129 x 33 loses (277 us a step against 262 in plain order)
+// where 41 x 129 x 41 gains 8%; most boxes gain. The mixed form loses much earlier
 // (per step: 17 x 65 x 17 174 against 216 us, 33 x 65 x 33 214 / 221, 49 x 33 x 49
 // 188 / 205, but 49 x 65 x 49 324 / 311, 33 x 97 x 33 277 / 272, 49 x 97 x 49 442 /
 // 402, 97 x 97 x 97 1105 / 1080): its line lies between 79 and 106 thousand entries.

@@ -20,7 +20,7 @@
 // as plain dot products and that column as an outer product, which beats padding
 // 65 to 72.
 // Bound: the FP64 tensor pipe (44 us of 79 for the three products back from the
-// eigenbasis at 129 x 129 columns, Ny = 129, pipe 60% active); the rest is the
+// eigenbasis at 129 x 129 columns, Ny = 129; pipe 56 to 67% active); the rest is the
 // stretch between two tiles of a CTA that the other CTA of the SM only partly
 // fills. Whole-operator tiles (k_dgemm_t) take 126 us for the same call, 103
 // against 67 us for the y-derivatives of two fields.

@@ -667,7 +667,7 @@ constexpr int kEigBatch = 4;    // rows whose loads are issued together (loads i
 // The FP64 form runs eight parts: half as long a chain of rows per thread, which
 // is the whole time of a small box (9 x 65 x 5 modes 8.8 us with the mean flow,
 // 13.5 + 6 us with four parts and a launch of its own; 129 x 129 x 129, bound by
-// HBM at 57 us, 73 against 70 + 9). The mixed form keeps four: another grouping
+// HBM at 57 us, 6 us less than two launches, 82 us in the step). The mixed form keeps four: another grouping
 // of the influence sums moves its rounding.
 constexpr int kEigParts64 = 8;
 // ... up to Ny = 202, where two blocks of eight parts (two kept arrays, 512 bytes

@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __res
 //  * c_inv enters once, squared, at the end instead of scaling every line.
 // Lane policies: a line on S lanes (S points each), or, where 16 S registers
 // do not fit, on 2 S lanes (S / 2 points each, sq2p_fft).
-// Bound: shared-memory wavefronts (65% of the pipe at 129 x 129 modes, 129
+// Bound: shared-memory wavefronts (67% of the pipe at 129 x 129 modes, 129
 // planes, S = 14; FP64 pipe 34%, HBM 15%). Measured there 240 us, 344 us with
 // seven arrays live, lanes (t, h) at t + S h and branches on the mode range;
 // 33 x 33 modes x 776 planes (S = 7) 85 us from 163, 49 x 49 x 65 24 from 49
@@ -884,7 +884,9 @@ __global__ void __launch_bounds__(kSqWarps * 32) k_xmid_h2(Geo g, const C* __res
 template <int S_>
 struct LineFull {
   static constexpr int S = S_, R = S, L = S, G = 32 / L, XB = sq_xbuf<S>(), TAB = S * sq_tw_stride(S);
-  // registers per thread: 4 arrays, the line and its temporaries (16 S + 20)
+  // Registers per thread: 4 arrays, the line and its temporaries. Caps of 128 (four
+  // blocks), 168 (three) and 255: S = 9 spills 108 bytes at 168, 7 32, 4 and 5 8;
+  // sides 3, 6, 8 and 10 none.
   static constexpr int BLOCKS = S <= 5 ? 4 : S <= 9 ? 3 : 2;
   static __device__ __forceinline__ int column(int li) { return li; }
   static __device__ __forceinline__ int half(int) { return 0; }
@@ -913,7 +915,7 @@ template <int S_>
 struct LineHalf {
   using Q = Sq2p<S_>;
   static constexpr int S = S_, R = S / 2, L = 2 * S, G = 32 / L, XB = Q::xbuf(), TAB = Q::tab();
-  static constexpr int BLOCKS = 3;
+  static constexpr int BLOCKS = 3;  // 168 registers: S = 14 fits, 12 spills 4 bytes, 16 56
   static __device__ __forceinline__ int column(int li) { return li >> 1; }
   static __device__ __forceinline__ int half(int li) { return li & 1; }
   static __device__ __forceinline__ int pos(int t, int h, int r) {

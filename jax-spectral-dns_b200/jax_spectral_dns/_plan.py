@@ -402,7 +402,7 @@ class GraphedSteps:
     """n_steps of a plan on fixed device buffers captured in one CUDA graph.
 
     ``jsd_step`` launches only on the caller's stream and allocates nothing,
-    so the whole loop (33 launches per step at the benchmark size) is recorded
+    so the whole loop (27 launches per step at the benchmark size) is recorded
     once and replayed with a single launch. The captured buffers (state,
     dpdx, the optional trajectory output and any registered dual history)
     must stay alive and in place; ``replay`` advances them exactly as the
